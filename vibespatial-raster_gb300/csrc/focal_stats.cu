@@ -35,8 +35,9 @@
 #include <cmath>
 #include <type_traits>
 
-#include "vsr_internal.cuh"
+#include "focal_stats.cuh"
 #include "std_round.h"
+#include "warp_strip.cuh"
 
 namespace vsr {
 namespace {
@@ -44,19 +45,6 @@ namespace {
 constexpr int kFsTX = 64, kFsTY = 16, kFsThreads = 256;
 constexpr int kFsMaxRadius = 31;        // window up to 63 x 63
 constexpr int kFsMaxVarietyRadius = 7;  // window up to 15 x 15 (225 taps)
-
-struct FsArgs {
-  const void* src;
-  int dtype;
-  int64_t H, W, pitch, band_stride;
-  int kind;     // resolved VSR_NODATA_*
-  double ndv;   // nodata in the element type (exact)
-  int ry, rx;
-  double nd_out;  // written for nodata centres and empty windows
-  void* dst;
-  int out_dtype;
-  int64_t out_pitch, out_band_stride;
-};
 
 template <typename T>
 __device__ __forceinline__ T pos_inf();
@@ -88,15 +76,6 @@ __device__ __forceinline__ double max_nan(double a, double b) { return (a != a |
 __device__ __forceinline__ void fs_store(const FsArgs& a, char* obase, int64_t idx, double v) {
   if (a.out_dtype == VSR_F64) reinterpret_cast<double*>(obase)[idx] = v;
   else reinterpret_cast<float*>(obase)[idx] = static_cast<float>(v);
-}
-
-// Nodata test in the element type itself (the value is exact there).
-template <typename TIN>
-__device__ __forceinline__ bool is_nd(TIN v, int kind, TIN ndv) {
-  if constexpr (std::is_floating_point<TIN>::value)
-    return kind == VSR_NODATA_VALUE ? v == ndv : (kind == VSR_NODATA_NAN ? v != v : false);
-  else
-    return kind == VSR_NODATA_VALUE && v == ndv;
 }
 
 // Staged value of one tap for statistic S (placeholder for nodata and
@@ -166,7 +145,7 @@ __global__ void __launch_bounds__(kFsThreads) focal_stat_kernel(const FsArgs a) 
     for (int c = lane; c < SW; c += 32) {
       const bool inb = row_in && c >= c_lo && c < c_hi;
       const TIN v = inb ? __ldg(rowp + c) : TIN(0);
-      const bool nd = inb && is_nd<TIN>(v, kind, ndv);
+      const bool nd = inb && fs_is_nd<TIN>(v, kind, ndv);
       St[r * SW + c] = staged<T, S, TIN>(inb && !nd, v);
       if (centre_row && c >= rx && c < rx + kFsTX) ndc[(r - ry) * kFsTX + (c - rx)] = nd;
     }
@@ -466,9 +445,14 @@ __global__ void __launch_bounds__(32 * kFwWarps) fs_warp_kernel(const FsArgs a) 
           }
           if constexpr (F64) {
             double* op = reinterpret_cast<double*>(obase) + orow;
+            if (VOUT && xs + 3 < a.W) {
+              store_32b(op, __double_as_longlong(qd[0]), __double_as_longlong(qd[1]), __double_as_longlong(qd[2]),
+                        __double_as_longlong(qd[3]));
+            } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (xs + c < a.W) op[c] = qd[c];
+              for (int c = 0; c < 4; ++c)
+                if (xs + c < a.W) op[c] = qd[c];
+            }
           } else {
             float* op = reinterpret_cast<float*>(obase) + orow;
             if (VOUT && xs + 3 < a.W) {
@@ -622,7 +606,7 @@ __global__ void __launch_bounds__(32 * kFwWarps) fs_warp_std(const FsArgs a) {
           s2 += wl[j];
         }
         float q[4];
-        double qd[4];
+        uint64_t qd[4];  // float64 bits
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           if (c > 0) {
@@ -634,14 +618,20 @@ __global__ void __launch_bounds__(32 * kFwWarps) fs_warp_std(const FsArgs a) {
           const uint64_t sq = (static_cast<uint64_t>(s1) << 16) + s2;
           const uint64_t N = static_cast<uint64_t>(cnt) * sq - static_cast<uint64_t>(sum) * sum;  // n^2 var
           const bool ok = (cm >> c) & 1u;  // a valid centre: cnt >= 1
-          if constexpr (F64) qd[c] = ok ? sqrt(static_cast<double>(N)) / cnt : a.nd_out;
+          if constexpr (F64)
+            qd[c] = !ok ? static_cast<uint64_t>(__double_as_longlong(a.nd_out))
+                        : (N ? vsr_s64_std(N, 0, fs_recip(cnt), 31 - __clz(cnt)) : 0ull);
           else q[c] = ok ? vsr_std_f32_small(N, cnt) : static_cast<float>(a.nd_out);
         }
         if constexpr (F64) {
           double* op = reinterpret_cast<double*>(obase) + orow;
+          if (VOUT && xs + 3 < a.W) {
+            store_32b(op, qd[0], qd[1], qd[2], qd[3]);
+          } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (xs + c < a.W) op[c] = qd[c];
+            for (int c = 0; c < 4; ++c)
+              if (xs + c < a.W) op[c] = __longlong_as_double(static_cast<long long>(qd[c]));
+          }
         } else {
           float* op = reinterpret_cast<float*>(obase) + orow;
           if (VOUT && xs + 3 < a.W) {
@@ -665,14 +655,16 @@ int fs_warp_launch(const FsArgs& a, int bands, cudaStream_t st) {
   const dim3 grid(static_cast<unsigned>((a.W + kFwWarps * kFwCols - 1) / (kFwWarps * kFwCols)),
                   static_cast<unsigned>((a.H + kFwStrip - 1) / kFwStrip), static_cast<unsigned>(bands));
   if (grid.y > 65535u) return -1;
-  const bool vout = a.out_dtype == VSR_F32 && aligned(a.dst, 16) && a.out_pitch % 4 == 0 &&
+  const bool vout = aligned(a.dst, a.out_dtype == VSR_F64 ? 32 : 16) && a.out_pitch % 4 == 0 &&
                     (bands == 1 || a.out_band_stride % 4 == 0);
   if constexpr (S == VSR_STAT_STD) {
-    if (a.out_dtype == VSR_F64) fs_warp_std<R, T, false, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
+    if (a.out_dtype == VSR_F64 && vout) fs_warp_std<R, T, true, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
+    else if (a.out_dtype == VSR_F64) fs_warp_std<R, T, false, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
     else if (vout) fs_warp_std<R, T, true, false><<<grid, 32 * kFwWarps, 0, st>>>(a);
     else fs_warp_std<R, T, false, false><<<grid, 32 * kFwWarps, 0, st>>>(a);
   } else {
-    if (a.out_dtype == VSR_F64) fs_warp_kernel<R, T, S, false, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
+    if (a.out_dtype == VSR_F64 && vout) fs_warp_kernel<R, T, S, true, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
+    else if (a.out_dtype == VSR_F64) fs_warp_kernel<R, T, S, false, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
     else if (vout) fs_warp_kernel<R, T, S, true, false><<<grid, 32 * kFwWarps, 0, st>>>(a);
     else fs_warp_kernel<R, T, S, false, false><<<grid, 32 * kFwWarps, 0, st>>>(a);
   }
@@ -718,6 +710,7 @@ int fs_dispatch(const FsArgs& a, int bands, cudaStream_t st) {
       case VSR_U16: rc = fs_warp_try<uint16_t, S>(a, bands, st); break;
       default: break;
     }
+    if (rc < 0) rc = fs_std_strip(a, bands, st);
     if (rc >= 0) return rc;
     switch (a.dtype) {
       case VSR_U8: return fs_launch<uint8_t, int32_t, S>(a, bands, st);
