@@ -310,7 +310,7 @@ __device__ __noinline__ void slow_strip(const FsArgs& a, const SdStrip& S) {
 }
 
 template <int R, typename T>
-__global__ void __launch_bounds__(kSdThreads) fs_strip_std(const FsArgs a, const int strip, const bool vin,
+__global__ void __launch_bounds__(kSdThreads, 5) fs_strip_std(const FsArgs a, const int strip, const bool vin,
                                                            const bool vout) {
   using G = SdGeom<R>;
   constexpr bool kFloat = std::is_same<T, float>::value;
@@ -392,10 +392,11 @@ int launch_strip_std(const FsArgs& a, int bands, cudaStream_t st) {
   auto kern = fs_strip_std<R, T>;
   VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   const int64_t gx = (a.W + kSdWarps * G::kCols - 1) / (kSdWarps * G::kCols);
-  // rows per strip: 64 (2R of them are read again by the next strip), 32
-  // where that would leave SMs without four blocks
-  int strip = 64;
-  if (gx * ((a.H + strip - 1) / strip) * bands < 4 * static_cast<int64_t>(sm_count())) strip = 32;
+  // rows per strip: the most that leaves two blocks per SM (2R rows of a strip
+  // are read again by the next one; 8192 x 4096, R = 3: 343 us at 128 rows,
+  // 380 us at 64; 4096 x 4096 the same at both)
+  int strip = 128;
+  while (strip > 16 && gx * ((a.H + strip - 1) / strip) * bands < 2 * static_cast<int64_t>(sm_count())) strip /= 2;
   const int64_t gy = (a.H + strip - 1) / strip;
   if (gy > 65535) return -1;
   const bool vin = aligned(a.src, 4 * sizeof(T)) && a.pitch % 4 == 0 && (bands == 1 || a.band_stride % 4 == 0);
