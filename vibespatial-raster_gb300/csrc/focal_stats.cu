@@ -1,5 +1,5 @@
 // Focal statistics other than the mean: min, max, range, std and variety
-// (the mean is focal.cu's exact box kernels).
+// (the mean is focal.cu's exact box kernels; variety is focal_variety.cu's).
 //
 // Semantics are the reference CPU functions' (algebra.py:3041-3164, run per
 // window by scipy generic_filter with out-of-bounds taps set to the
@@ -27,10 +27,10 @@
 // int32 for the integer std), nodata and out-of-bounds taps already replaced
 // by the statistic's placeholder.  min / max / range are separable: a row
 // pass reduces each staged row to 64 window rows in shared memory, the
-// column pass reduces 2ry+1 of those.  std and variety run over the staged
-// window per pixel: std as exact int64 sums for 8/16-bit rasters
-// (var = (n sum x^2 - (sum x)^2) / n^2) and two passes in float64 otherwise;
-// variety counts the taps with no equal earlier tap.  Bands are blockIdx.z.
+// column pass reduces 2ry+1 of those.  std runs as exact separable int64 sums
+// for 8/16-bit rasters (var = (n sum x^2 - (sum x)^2) / n^2) and over the
+// staged window per pixel, two passes in float64, otherwise -- what
+// focal_std.cu does not take.  Bands are blockIdx.z.
 #include <cfloat>
 #include <cmath>
 #include <type_traits>
@@ -44,7 +44,6 @@ namespace {
 
 constexpr int kFsTX = 64, kFsTY = 16, kFsThreads = 256;
 constexpr int kFsMaxRadius = 31;        // window up to 63 x 63
-constexpr int kFsMaxVarietyRadius = 7;  // window up to 15 x 15 (225 taps)
 
 template <typename T>
 __device__ __forceinline__ T pos_inf();
@@ -114,7 +113,7 @@ struct FsLayout {  // shared-memory carve-up of one CTA (byte offsets)
 // in the statistic's type with placeholders applied, and the centre
 // pixels' nodata flags.  min / max / range and the 8/16-bit std are
 // separable (a row pass into shared memory, a column pass); the float std
-// (two float64 passes) and variety run over the staged window per pixel.
+// (two float64 passes) runs over the staged window per pixel.
 template <typename TIN, typename T, int S>
 __global__ void __launch_bounds__(kFsThreads) focal_stat_kernel(const FsArgs a) {
   using Lay = FsLayout<S, T>;
@@ -240,45 +239,27 @@ __global__ void __launch_bounds__(kFsThreads) focal_stat_kernel(const FsArgs a) 
     for (int r = warp; r < nr; r += WARPS)
       for (int c = lane; c < nc; c += 32) {
         const T* win = St + r * SW + c;
-        double out;
-        if constexpr (S == VSR_STAT_STD) {
-          double sm = 0.0;
-          int n = 0;
+        double sm = 0.0;
+        int n = 0;
+        for (int dy = 0; dy < kh; ++dy)
+          for (int dx = 0; dx < kw; ++dx) {
+            const double v = win[dy * SW + dx];
+            if (v != v) continue;
+            sm += v;
+            ++n;
+          }
+        double m2 = 0.0;
+        if (n) {
+          const double mean = sm / n;
           for (int dy = 0; dy < kh; ++dy)
             for (int dx = 0; dx < kw; ++dx) {
               const double v = win[dy * SW + dx];
               if (v != v) continue;
-              sm += v;
-              ++n;
+              const double d = v - mean;
+              m2 = fma(d, d, m2);
             }
-          double m2 = 0.0;
-          if (n) {
-            const double mean = sm / n;
-            for (int dy = 0; dy < kh; ++dy)
-              for (int dx = 0; dx < kw; ++dx) {
-                const double v = win[dy * SW + dx];
-                if (v != v) continue;
-                const double d = v - mean;
-                m2 = fma(d, d, m2);
-              }
-          }
-          out = n ? sqrt(m2 / n) : 0.0;
-        } else {  // variety: taps with no equal earlier tap
-          int cnt = 0;
-          for (int iy = 0; iy < kh; ++iy)
-            for (int ix = 0; ix < kw; ++ix) {
-              const T v = win[iy * SW + ix];
-              if (v != v) continue;
-              bool dup = false;
-              for (int jy = 0; jy <= iy && !dup; ++jy) {
-                const int jend = jy < iy ? kw : ix;
-                for (int jx = 0; jx < jend; ++jx)
-                  if (win[jy * SW + jx] == v) { dup = true; break; }
-              }
-              cnt += !dup;
-            }
-          out = cnt;
         }
+        const double out = n ? sqrt(m2 / n) : 0.0;
         out_at(r, c, out);
       }
   }
@@ -721,16 +702,14 @@ int fs_dispatch(const FsArgs& a, int bands, cudaStream_t st) {
       default: return fs_launch<double, double, S>(a, bands, st);
     }
   } else {
-    if constexpr (S != VSR_STAT_VARIETY) {
-      int rc = -1;
-      switch (a.dtype) {
-        case VSR_U8: rc = fs_warp_try<uint8_t, S>(a, bands, st); break;
-        case VSR_I16: rc = fs_warp_try<int16_t, S>(a, bands, st); break;
-        case VSR_U16: rc = fs_warp_try<uint16_t, S>(a, bands, st); break;
-        default: break;
-      }
-      if (rc >= 0) return rc;
+    int rc = -1;
+    switch (a.dtype) {
+      case VSR_U8: rc = fs_warp_try<uint8_t, S>(a, bands, st); break;
+      case VSR_I16: rc = fs_warp_try<int16_t, S>(a, bands, st); break;
+      case VSR_U16: rc = fs_warp_try<uint16_t, S>(a, bands, st); break;
+      default: break;
     }
+    if (rc >= 0) return rc;
     switch (a.dtype) {
       case VSR_U8: return fs_launch<uint8_t, float, S>(a, bands, st);
       case VSR_I16: return fs_launch<int16_t, float, S>(a, bands, st);
@@ -798,7 +777,7 @@ extern "C" int vsr_focal_stat_bands(const void* src, int dtype, int bands, int64
     case VSR_STAT_MAX: return fs_dispatch<VSR_STAT_MAX>(a, bands, st);
     case VSR_STAT_STD: return fs_dispatch<VSR_STAT_STD>(a, bands, st);
     case VSR_STAT_RANGE: return fs_dispatch<VSR_STAT_RANGE>(a, bands, st);
-    default: return fs_dispatch<VSR_STAT_VARIETY>(a, bands, st);
+    default: return fs_variety(a, bands, st);
   }
 }
 

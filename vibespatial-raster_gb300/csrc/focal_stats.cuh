@@ -10,6 +10,8 @@
 
 namespace vsr {
 
+constexpr int kFsMaxVarietyRadius = 7;  // window up to 15 x 15 (225 taps)
+
 struct FsArgs {
   const void* src;
   int dtype;
@@ -47,5 +49,6 @@ __device__ __forceinline__ uint64_t fs_recip(uint32_t n) { return __ldg(&g_recip
 
 // Launch the kernel if it serves these arguments; -1 otherwise.
 int fs_std_strip(const FsArgs& a, int bands, cudaStream_t st);  // focal_std.cu
+int fs_variety(const FsArgs& a, int bands, cudaStream_t st);    // focal_variety.cu: every dtype and window
 
 }  // namespace vsr
