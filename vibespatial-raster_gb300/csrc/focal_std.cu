@@ -1,6 +1,5 @@
-// Focal standard deviation with exact integer sums: float32 rasters and the
-// 8/16-bit ones that fs_warp_std (focal_stats.cu) does not take (rows not
-// aligned to 4 elements, radius 5 to 7), square windows of radius 1..7.
+// Focal standard deviation with exact integer sums: 8/16-bit and float32
+// rasters, square windows of radius 1..7.
 //
 // The reference takes two float64 passes over every window (algebra.py:
 // 3104-3122).  An SM of a GB300 starts only two FP64 operations per clock, so
@@ -24,8 +23,10 @@
 // of integers wait in shared memory, each thread reading only its own), takes
 // the column sums of its neighbours by shuffles and adds up the window.
 //
-// Bound by instruction issue (about 130 per pixel, 70 of them the square root
-// and division).
+// Bound by instruction issue (about 150 per pixel, half of them the square
+// root and division).  7 x 7 on 4096^2: float32 151 us (8370 us with the two
+// float64 passes), uint16 128 us and 205 us with a float32 output (404 and
+// 586 us in 256-row strips of 128 threads with an FP64 root).
 #include <cstring>
 
 #include "focal_stats.cuh"
@@ -35,8 +36,7 @@
 namespace vsr {
 namespace {
 
-constexpr int kSdWarps = 4;
-constexpr int kSdThreads = 32 * kSdWarps;
+constexpr int kSdThreads = 32;  // one warp per block: blocks of unequal strips (one word, two limbs) balance best
 constexpr int kSdMaxR = 7;  // windows of at most kRecipTaps: a count fits a byte
 static_assert((2 * kSdMaxR + 1) * (2 * kSdMaxR + 1) <= kRecipTaps, "reciprocal table");
 
@@ -122,17 +122,20 @@ struct SdStrip {
   int64_t xw, ys;  // first column of lane 0, first output row
   int nout;
   int u;           // values are integers times 2^u
+  bool inside;     // all 128 columns lie in the raster
+  float ndq;       // float32 rasters: the nodata value, or NaN (equal to nothing)
   float s1, s2;    // float32 rasters: value * s1 = its integer; s2 = s1 2^-kLB
   int ref;         // subtracted from the integers (one word)
 };
 
-template <int R, typename T, int LIMBS>
+template <int R, typename T, int LIMBS, bool EDGE>
 __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, bool vin, bool vout, int4* ring,
                                           uint32_t* flags, uint64_t* obuf) {
   using G = SdGeom<R>;
   constexpr int P = G::P;
   constexpr bool kFloat = std::is_same<T, float>::value;
   const int lane = threadIdx.x & 31, t = threadIdx.x;
+  const bool has_nd = a.kind != VSR_NODATA_NONE, nd_nan = a.kind == VSR_NODATA_NAN;
   const T ndv = static_cast<T>(a.ndv);
   const int64_t xs = S.xw + 4 * lane;
   uint32_t inm = 0;
@@ -142,16 +145,18 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
   const T* lp = src + (S.ys - R) * a.pitch + xs;
   const int nin = S.nout + 2 * R;
   auto row_in = [&](int i) { return static_cast<uint64_t>(S.ys - R + i) < static_cast<uint64_t>(a.H); };
+  ring += t;
+  flags += t;
   for (int s = 0; s < P; ++s) {
 #pragma unroll
-    for (int l = 0; l < LIMBS; ++l) ring[(s * LIMBS + l) * kSdThreads + t] = make_int4(0, 0, 0, 0);
-    flags[s * kSdThreads + t] = 0u;
+    for (int l = 0; l < LIMBS; ++l) ring[(s * LIMBS + l) * kSdThreads] = make_int4(0, 0, 0, 0);
+    flags[s * kSdThreads] = 0u;
   }
   int32_t sh[4] = {0, 0, 0, 0}, sl[4] = {0, 0, 0, 0};
   uint64_t qh[4] = {0, 0, 0, 0}, qm[4] = {0, 0, 0, 0}, ql[4] = {0, 0, 0, 0};
   uint32_t cw = 0;
-  uint32_t nxt[4];
-  strip_load4<T>(lp, row_in(0) ? inm : 0u, vin, nxt);
+  uint32_t nxt[4] = {0u, 0u, 0u, 0u};
+  if (row_in(0)) strip_load4<T, EDGE>(lp, inm, vin, nxt);
   const int64_t xo = S.xw;
   constexpr int lo = 4 * G::HL;
   const int hi = static_cast<int>(a.W - xo < 128 - 4 * G::HL ? a.W - xo : static_cast<int64_t>(128 - 4 * G::HL));
@@ -161,38 +166,45 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
   int slot = 0, cslot = P - R;
 #pragma unroll 1
   for (int i = 0; i < nin; ++i) {
-    uint32_t raw[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) raw[e] = nxt[e];
-    const uint32_t in = row_in(i) ? inm : 0u;
-    lp += a.pitch;
-    strip_load4<T>(lp, i + 1 < nin && row_in(i + 1) ? inm : 0u, vin, nxt);
     // integers of the entering row
-    int32_t nh[4], nl[4];
-    uint32_t f = 0;
+    int32_t nh[4] = {0, 0, 0, 0}, nl[4] = {0, 0, 0, 0};
+    uint32_t f = 0;  // byte e: 1 valid, 2 nodata
+    if (row_in(i)) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const T v = elem_of<T>(raw[e]);
-      const bool ib = (in >> e) & 1u, nd = ib && fs_is_nd<T>(v, a.kind, ndv);
-      const bool ok = ib && !nd && v == v;
-      f |= (ok ? 1u : 0u) << (8 * e) | (nd ? 2u : 0u) << (8 * e);
-      if constexpr (!kFloat) {
-        nh[e] = ok ? static_cast<int32_t>(v) : 0;
-      } else if constexpr (LIMBS == 1) {
-        nh[e] = ok ? __float2int_rn(v * S.s1) - S.ref : 0;
-      } else {
-        // v = h 2^kLB + l (units), both of v's sign; the remainder is exact
-        const float q = ok ? v * S.s2 : 0.0f;
-        const float qt = truncf(q);
-        nh[e] = __float2int_rz(qt);
-        nl[e] = __float2int_rn((q - qt) * static_cast<float>(1 << G::kLB));
+      for (int e = 0; e < 4; ++e) {
+        const T v = elem_of<T>(nxt[e]);
+        bool nd, ok;
+        if constexpr (kFloat) {
+          const bool eq = v == S.ndq;
+          ok = !eq && v == v;
+          nd = nd_nan ? v != v : eq;
+        } else {
+          nd = has_nd && v == ndv;
+          ok = !nd;
+        }
+        if (EDGE) ok = ok && ((inm >> e) & 1u);  // nd outside the raster: never a centre that is written
+        f |= ok ? 1u << (8 * e) : 0u;
+        f |= nd ? 2u << (8 * e) : 0u;
+        if constexpr (!kFloat) {
+          nh[e] = ok ? static_cast<int32_t>(v) : 0;
+        } else if constexpr (LIMBS == 1) {
+          nh[e] = ok ? __float2int_rn(v * S.s1) - S.ref : 0;
+        } else {
+          // v = h 2^kLB + l (units), both of v's sign; the remainder is exact
+          const float q = ok ? v * S.s2 : 0.0f;
+          const float qt = truncf(q);
+          nh[e] = __float2int_rz(qt);
+          nl[e] = __float2int_rn((q - qt) * static_cast<float>(1 << G::kLB));
+        }
       }
     }
-    const int4 oh = ring[(slot * LIMBS) * kSdThreads + t];
-    ring[(slot * LIMBS) * kSdThreads + t] = make_int4(nh[0], nh[1], nh[2], nh[3]);
+    lp += a.pitch;
+    if (i + 1 < nin && row_in(i + 1)) strip_load4<T, EDGE>(lp, inm, vin, nxt);
+    const int4 oh = ring[(slot * LIMBS) * kSdThreads];
+    ring[(slot * LIMBS) * kSdThreads] = make_int4(nh[0], nh[1], nh[2], nh[3]);
     const int32_t ph[4] = {oh.x, oh.y, oh.z, oh.w};
-    const uint32_t fo = flags[slot * kSdThreads + t];
-    flags[slot * kSdThreads + t] = f;
+    const uint32_t fo = flags[slot * kSdThreads];
+    flags[slot * kSdThreads] = f;
     cw += (f & 0x01010101u) - (fo & 0x01010101u);
     if constexpr (LIMBS == 1) {
 #pragma unroll
@@ -202,8 +214,8 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
         qh[e] += static_cast<uint64_t>(static_cast<int64_t>(-ph[e]) * ph[e]);
       }
     } else {
-      const int4 ol = ring[(slot * LIMBS + 1) * kSdThreads + t];
-      ring[(slot * LIMBS + 1) * kSdThreads + t] = make_int4(nl[0], nl[1], nl[2], nl[3]);
+      const int4 ol = ring[(slot * LIMBS + 1) * kSdThreads];
+      ring[(slot * LIMBS + 1) * kSdThreads] = make_int4(nl[0], nl[1], nl[2], nl[3]);
       const int32_t pl[4] = {ol.x, ol.y, ol.z, ol.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -230,7 +242,7 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
         window4<R>(qm, wqm);
         window4<R>(ql, wql);
       }
-      const uint32_t fc = flags[cslot * kSdThreads + t];  // the centre row i - R
+      const uint32_t fc = flags[cslot * kSdThreads];  // the centre row i - R
       uint64_t o64[4];
       uint32_t o32[4];
 #pragma unroll
@@ -309,49 +321,61 @@ __device__ __noinline__ void slow_strip(const FsArgs& a, const SdStrip& S) {
   }
 }
 
+// Range of the strip's valid values, halo included.
+template <int R, bool EDGE>
+__device__ __forceinline__ void scan_range(const FsArgs& a, const SdStrip& S, bool vin, uint32_t& amin, float& vmin,
+                                           float& vmax) {
+  const int64_t xs = S.xw + 4 * (threadIdx.x & 31);
+  uint32_t inm = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) inm |= static_cast<uint32_t>(xs + e >= 0 && xs + e < a.W) << e;
+  const int64_t g0 = S.ys - R < 0 ? 0 : S.ys - R, g1 = S.ys + S.nout + R < a.H ? S.ys + S.nout + R : a.H;
+  const int rows = static_cast<int>(g1 - g0);
+  const float* lp = static_cast<const float*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride +
+                    g0 * a.pitch + xs;
+#pragma unroll 4
+  for (int i = 0; i < rows; ++i, lp += a.pitch) {
+    uint32_t raw[4];
+    strip_load4<float, EDGE>(lp, inm, vin, raw);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float v = __uint_as_float(raw[e]);
+      bool ok = v != S.ndq && v == v;
+      if (EDGE) ok = ok && ((inm >> e) & 1u);
+      amin = min(amin, ok ? (raw[e] & 0x7fffffffu) - 1u : 0xFFFFFFFFu);
+      vmin = fminf(vmin, ok ? v : __int_as_float(0x7f800000));
+      vmax = fmaxf(vmax, ok ? v : __int_as_float(0xff800000));
+    }
+  }
+}
+
+// 16 blocks per SM (128 registers); 20 blocks spill: a 7 x 7 std takes 143 us
+// against 153 at 4096^2 with them, but 65 against 55 at 1000 x 4096.
 template <int R, typename T>
-__global__ void __launch_bounds__(kSdThreads, 5) fs_strip_std(const FsArgs a, const int strip, const bool vin,
+__global__ void __launch_bounds__(kSdThreads, 16) fs_strip_std(const FsArgs a, const int strip, const bool vin,
                                                            const bool vout) {
   using G = SdGeom<R>;
   constexpr bool kFloat = std::is_same<T, float>::value;
   constexpr int kLimbs = kFloat ? 2 : 1;
   extern __shared__ __align__(16) unsigned char sd_smem[];
-  uint64_t* obuf = reinterpret_cast<uint64_t*>(sd_smem) + 128 * (threadIdx.x >> 5);
-  int4* ring = reinterpret_cast<int4*>(sd_smem + kSdWarps * 128 * 8);
+  uint64_t* obuf = reinterpret_cast<uint64_t*>(sd_smem);
+  int4* ring = reinterpret_cast<int4*>(sd_smem + 128 * 8);
   uint32_t* flags = reinterpret_cast<uint32_t*>(ring + G::P * kLimbs * kSdThreads);
   SdStrip S{};
-  S.xw = (static_cast<int64_t>(blockIdx.x) * kSdWarps + (threadIdx.x >> 5)) * G::kCols - 4 * G::HL;
-  if (S.xw + 4 * G::HL >= a.W) return;  // the whole warp: no block-wide barrier follows
+  S.xw = static_cast<int64_t>(blockIdx.x) * G::kCols - 4 * G::HL;
   S.ys = static_cast<int64_t>(blockIdx.y) * strip;
   S.nout = static_cast<int>(a.H - S.ys < strip ? a.H - S.ys : static_cast<int64_t>(strip));
+  S.inside = S.xw >= 0 && S.xw + 128 <= a.W;
   if constexpr (!kFloat) {
-    run_strip<R, T, 1>(a, S, vin, vout, ring, flags, obuf);
+    if (S.inside) run_strip<R, T, 1, false>(a, S, vin, vout, ring, flags, obuf);
+    else run_strip<R, T, 1, true>(a, S, vin, vout, ring, flags, obuf);
   } else {
     // smallest non-zero magnitude and range of the strip's valid values
-    const int lane = threadIdx.x & 31;
-    const int64_t xs = S.xw + 4 * lane;
-    uint32_t inm = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) inm |= static_cast<uint32_t>(xs + e >= 0 && xs + e < a.W) << e;
-    const float ndv = static_cast<float>(a.ndv);
-    const float* src = static_cast<const float*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride;
-    uint32_t amin = 0xFFFFFFFFu;
+    S.ndq = a.kind == VSR_NODATA_VALUE ? static_cast<float>(a.ndv) : __int_as_float(0x7fffffff);
+    uint32_t amin = 0xFFFFFFFFu;  // smallest non-zero magnitude's bits, less 1
     float vmin = __int_as_float(0x7f800000), vmax = -vmin;
-    const int64_t g0 = S.ys - R < 0 ? 0 : S.ys - R, g1 = S.ys + S.nout + R < a.H ? S.ys + S.nout + R : a.H;
-#pragma unroll 4
-    for (int64_t gy = g0; gy < g1; ++gy) {
-      uint32_t raw[4];
-      strip_load4<float>(src + gy * a.pitch + xs, inm, vin, raw);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float v = __uint_as_float(raw[e]);
-        const bool ok = ((inm >> e) & 1u) && !fs_is_nd<float>(v, a.kind, ndv) && v == v;
-        const uint32_t m = raw[e] & 0x7fffffffu;
-        amin = min(amin, ok && m ? m : 0xFFFFFFFFu);
-        vmin = fminf(vmin, ok ? v : vmin);
-        vmax = fmaxf(vmax, ok ? v : vmax);
-      }
-    }
+    if (S.inside) scan_range<R, false>(a, S, vin, amin, vmin, vmax);
+    else scan_range<R, true>(a, S, vin, amin, vmin, vmax);
 #pragma unroll
     for (int d = 16; d; d >>= 1) {
       amin = min(amin, __shfl_xor_sync(0xffffffffu, amin, d));
@@ -359,9 +383,10 @@ __global__ void __launch_bounds__(kSdThreads, 5) fs_strip_std(const FsArgs a, co
       vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, d));
     }
     if (amin == 0xFFFFFFFFu) {  // no value, or zeros only: any unit
-      amin = 0x3f800000u;
+      amin = 0x3f7fffffu;
       vmin = vmax = 0.0f;
     }
+    ++amin;
     const int E = static_cast<int>(amin >> 23);
     const float vabs = fmaxf(fabsf(vmin), fabsf(vmax));
     const int span = static_cast<int>(__float_as_uint(vabs) >> 23) - E;
@@ -377,9 +402,10 @@ __global__ void __launch_bounds__(kSdThreads, 5) fs_strip_std(const FsArgs a, co
     const float units = __fmul_ru(__fsub_ru(vmax, vmin), S.s1);
     if (span <= 6 && units < 4294900000.0f / static_cast<float>(G::kTaps)) {
       S.ref = __float2int_rn(vmin * S.s1) + __float2int_rn(0.5f * units);
-      run_strip<R, T, 1>(a, S, vin, vout, ring, flags, obuf);
+      if (S.inside) run_strip<R, T, 1, false>(a, S, vin, vout, ring, flags, obuf);
+      else run_strip<R, T, 1, true>(a, S, vin, vout, ring, flags, obuf);
     } else {
-      run_strip<R, T, 2>(a, S, vin, vout, ring, flags, obuf);
+      run_strip<R, T, 2, true>(a, S, vin, vout, ring, flags, obuf);
     }
   }
 }
@@ -388,15 +414,17 @@ template <int R, typename T>
 int launch_strip_std(const FsArgs& a, int bands, cudaStream_t st) {
   using G = SdGeom<R>;
   constexpr int kLimbs = std::is_same<T, float>::value ? 2 : 1;
-  const size_t smem = kSdWarps * 128 * 8 + static_cast<size_t>(G::P) * kSdThreads * (16 * kLimbs + 4);
+  const size_t smem = 128 * 8 + static_cast<size_t>(G::P) * kSdThreads * (16 * kLimbs + 4);
   auto kern = fs_strip_std<R, T>;
-  VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  const int64_t gx = (a.W + kSdWarps * G::kCols - 1) / (kSdWarps * G::kCols);
-  // rows per strip: the most that leaves two blocks per SM (2R rows of a strip
-  // are read again by the next one; 8192 x 4096, R = 3: 343 us at 128 rows,
-  // 380 us at 64; 4096 x 4096 the same at both)
+  static KernelResidency residency;
+  int per_sm = 0;
+  VSR_CUDA_TRY(residency.get(kern, kSdThreads, smem, &per_sm));
+  const int64_t gx = (a.W + G::kCols - 1) / G::kCols;
+  // rows per strip: the most that leaves every SM 32 blocks, two rounds of
+  // what fits (2R rows of a strip are read again by the next one).  4096^2,
+  // 11 x 11: 178 us with that, 191 us with 16 blocks per SM
   int strip = 128;
-  while (strip > 16 && gx * ((a.H + strip - 1) / strip) * bands < 2 * static_cast<int64_t>(sm_count())) strip /= 2;
+  while (strip > 16 && gx * ((a.H + strip - 1) / strip) * bands < 32 * static_cast<int64_t>(sm_count())) strip /= 2;
   const int64_t gy = (a.H + strip - 1) / strip;
   if (gy > 65535) return -1;
   const bool vin = aligned(a.src, 4 * sizeof(T)) && a.pitch % 4 == 0 && (bands == 1 || a.band_stride % 4 == 0);

@@ -1,10 +1,11 @@
 // Focal variety: the number of distinct valid values in the window
 // (semantics of algebra.py:3146-3163; no cap on the count).
 //
-// Two forms.
+// Two forms (on a 5001 x 4999 map of 12 classes and holes, 5 x 5: 92 us, 2.4
+// TB/s, against 2680 us for comparing all pairs of taps).
 //
 // * fs_variety_bits -- 8/16-bit rasters, square windows of radius 1..7.  A
-//   block finds the set of values of its 480 x 64 tile (with the halo) and
+//   block finds the set of values of its tile (with the halo) and
 //   numbers them; a window's set is then the OR of its pixels' one-hot words,
 //   which is separable: rows first (neighbours' words by shuffles, the
 //   layout of warp_strip.cuh), then the last 2R+1 rows' results, which wait
@@ -31,10 +32,11 @@
 namespace vsr {
 namespace {
 
-constexpr int kVyWarps = 4, kVyThreads = 32 * kVyWarps;
+constexpr int kVyThreads = 128;      // block of the pairs form
 constexpr int kVyMaxR = 7;           // nibbles: 2 r + 1 <= 15 columns, dy <= 14
 constexpr int kVyTX = 64, kVyTY = 16;  // tile of the pairs form
-constexpr int kVyStrip = 64;         // rows of a block of the bits form
+constexpr int kVyStrip = 16;         // rows of a block of the bits form
+constexpr int kVyOut = 258;          // output table: counts 0 .. 225, nodata at 256
 
 __device__ __forceinline__ void vy_store(const FsArgs& a, int64_t o, double v) {
   if (a.out_dtype == VSR_F64) static_cast<double*>(a.dst)[o] = v;
@@ -69,7 +71,7 @@ __host__ __device__ inline size_t vy_pairs_smem(int ry, int rx) {
 // One 64 x 16 tile at (x0, y0) of the block's band (columns below x1) by all
 // its threads.
 // R > 0: a square window of that radius; R == 0: the radii of ``a``.
-template <typename T, int R>
+template <typename T, int R, int THREADS>
 __device__ void variety_pairs(const FsArgs& a, int64_t x0, int64_t y0, int64_t x1, unsigned char* smem) {
   using K = VyKey<T>;
   const int ry = R ? R : a.ry, rx = R ? R : a.rx;
@@ -80,7 +82,7 @@ __device__ void variety_pairs(const FsArgs& a, int64_t x0, int64_t y0, int64_t x
   const int tid = threadIdx.x;
   const T* src = static_cast<const T*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride;
   const T ndv = static_cast<T>(a.ndv);
-  for (int i = tid; i < SH * SP; i += kVyThreads) {
+  for (int i = tid; i < SH * SP; i += THREADS) {
     const int r = i / SP, c = i - r * SP - 2 * rx;
     const int64_t gy = y0 - ry + r, gx = x0 - rx + c;
     K k = vy_none<K>();
@@ -96,7 +98,7 @@ __device__ void variety_pairs(const FsArgs& a, int64_t x0, int64_t y0, int64_t x
   }
   __syncthreads();
   const int kw = 2 * rx + 1;
-  for (int i = tid; i < SH * SW; i += kVyThreads) {
+  for (int i = tid; i < SH * SW; i += THREADS) {
     const int r = i / SW, c = i - r * SW;
     const K* p = key + r * SP + 2 * rx + c;
     const K k = *p;
@@ -130,7 +132,7 @@ __device__ void variety_pairs(const FsArgs& a, int64_t x0, int64_t y0, int64_t x
   __syncthreads();
   const int nr = static_cast<int>(a.H - y0 < kVyTY ? a.H - y0 : int64_t(kVyTY));
   const int nc = static_cast<int>(x1 - x0 < kVyTX ? x1 - x0 : int64_t(kVyTX));
-  for (int i = tid; i < kVyTX * kVyTY; i += kVyThreads) {
+  for (int i = tid; i < kVyTX * kVyTY; i += THREADS) {
     const int r = i / kVyTX, c = i - r * kVyTX;
     if (r >= nr || c >= nc) continue;
     int cnt = 0;
@@ -151,7 +153,7 @@ __device__ void variety_pairs(const FsArgs& a, int64_t x0, int64_t y0, int64_t x
 template <typename T, int R>
 __global__ void __launch_bounds__(kVyThreads) fs_variety_pairs(const FsArgs a) {
   extern __shared__ __align__(16) unsigned char vy_smem[];
-  variety_pairs<T, R>(a, static_cast<int64_t>(blockIdx.x) * kVyTX, static_cast<int64_t>(blockIdx.y) * kVyTY, a.W,
+  variety_pairs<T, R, kVyThreads>(a, static_cast<int64_t>(blockIdx.x) * kVyTX, static_cast<int64_t>(blockIdx.y) * kVyTY, a.W,
                       vy_smem);
 }
 
@@ -162,73 +164,219 @@ struct VyGeom {
   static constexpr int HL = (R + 3) / 4;
   static constexpr int kCols = 128 - 8 * HL;
   static constexpr bool kByte = sizeof(T) == 1;
+  // 4 warps share the value table; 16 rows per block keep its set small and
+  // the blocks many.  5001 x 4999, 5 x 5, rows x warps: 16 x 4 92 us, 32 x 4
+  // 94, 64 x 4 127, 32 x 2 92, 32 x 1 117; 400 values in 16 bits: 595, 672, 788
+  static constexpr int kWarps = 4, kThreads = 32 * kWarps;
   static constexpr int kMaxValues = kTaps * kTaps / 2;  // see above
-  // shared memory, in bytes: value table, transfer buffer, packed counts
-  // (several passes), the rows' words and nodata flags
+  // shared memory, in bytes: value table, output table, transfer buffer, the
+  // rows' words and nodata flags, packed counts (several passes)
   static constexpr int kTab = kByte ? 256 * 4 : 2048 * 8;
-  static constexpr int kBuf = kVyWarps * 128 * 8, kCnt = kVyStrip * kVyThreads * 4;
-  static constexpr int kRing = P * kVyThreads * 20;
-  static constexpr size_t smem() { return static_cast<size_t>(kTab) + kBuf + kCnt + kRing; }
+  static constexpr int kBuf = kWarps * 128 * 8, kCnt = kVyStrip * kThreads * 4;
+  static constexpr int kRing = P * kThreads * 20;
+  static constexpr size_t smem() { return static_cast<size_t>(kTab) + kVyOut * 8 + kBuf + kCnt + kRing; }
 };
 
+// A warp's strip of a block's tile.
+struct VyStrip {
+  int64_t xw, xs, ys;  // first column of lane 0, of this lane; first output row
+  int nout;
+  uint32_t inm;        // this lane's columns inside the raster
+  bool vin, vout, has_nd;
+  uint32_t ndk;        // nodata's bit pattern
+};
+
+// Mark the strip's values.  8-bit: a word per value (plain stores); 16-bit: a
+// bitmap, tested before the atomic (most pixels repeat a value).  Nodata is
+// taken out of the table afterwards.
+template <int R, typename T, bool EDGE>
+__device__ __forceinline__ void vy_scan(const FsArgs& a, const T* src, const VyStrip& S, uint32_t* lut, uint2* tab) {
+  const int64_t g0 = S.ys - R < 0 ? 0 : S.ys - R, g1 = S.ys + S.nout + R < a.H ? S.ys + S.nout + R : a.H;
+  const int rows = static_cast<int>(g1 - g0);
+  const T* lp = src + g0 * a.pitch + S.xs;
+#pragma unroll 4
+  for (int i = 0; i < rows; ++i, lp += a.pitch) {
+    uint32_t e4[4];
+    strip_load4<T, EDGE>(lp, S.inm, S.vin, e4);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const bool in = !EDGE || ((S.inm >> e) & 1u);
+      if (sizeof(T) == 1) {
+        if (in) lut[e4[e]] = 1u;
+      } else {
+        const uint32_t b = 1u << (e4[e] & 31u);
+        if (in && !(*reinterpret_cast<volatile uint32_t*>(&tab[e4[e] >> 5].x) & b)) atomicOr(&tab[e4[e] >> 5].x, b);
+      }
+    }
+  }
+}
+
+// One pass over the strip: the counts of values 32 w .. 32 w + 31, added to
+// those of the earlier passes (``cbuf``, unless the first); the last pass
+// writes the outputs through ``out``: the bits of count n at n, of nodata at
+// 256.
+template <int R, typename T, bool EDGE>
+__device__ __forceinline__ void vy_pass(const FsArgs& a, const T* src, const VyStrip& S, int w, bool last,
+                                        const uint32_t* lut, const uint2* tab, const uint64_t* out, uint32_t* cbuf,
+                                        uint4* ring, uint32_t* flags, uint64_t* obuf) {
+  using G = VyGeom<R, T>;
+  constexpr int P = G::P, HL = G::HL;
+  const int t = threadIdx.x, lane = t & 31;
+  const int nin = S.nout + 2 * R;
+  constexpr int lo = 4 * HL;
+  const int hi = static_cast<int>(a.W - S.xw < 128 - 4 * HL ? a.W - S.xw : static_cast<int64_t>(128 - 4 * HL));
+  const bool f64 = a.out_dtype == VSR_F64;
+  auto row_in = [&](int i) { return static_cast<uint64_t>(S.ys - R + i) < static_cast<uint64_t>(a.H); };
+  const T* lp = src + (S.ys - R) * a.pitch + S.xs;
+  uint32_t nxt[4] = {0u, 0u, 0u, 0u};
+  if (row_in(0)) strip_load4<T, EDGE>(lp, S.inm, S.vin, nxt);
+  int64_t orow = static_cast<int64_t>(blockIdx.z) * a.out_band_stride + S.ys * a.out_pitch + S.xw;
+  int slot = 0, cslot = P - R;
+#pragma unroll 1
+  for (int i = 0; i < nin; ++i) {
+    uint32_t o[4 * (2 * HL + 1)];
+    uint32_t f = 0;
+    if (row_in(i)) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint32_t word;
+        if (G::kByte) {
+          word = lut[nxt[e]];
+        } else {
+          const uint2 en = tab[nxt[e] >> 5];
+          const uint32_t b = 1u << (nxt[e] & 31u), rank = en.y + __popc(en.x & (b - 1u)) - 32u * w;
+          word = (en.x & b) && rank < 32u ? 1u << rank : 0u;
+        }
+        if (EDGE && !((S.inm >> e) & 1u)) word = 0u;
+        o[4 * HL + e] = word;
+      }
+      if (last && S.has_nd) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f |= nxt[e] == S.ndk ? 1u << e : 0u;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[4 * HL + e] = 0u;
+    }
+    lp += a.pitch;
+    if (i + 1 < nin && row_in(i + 1)) strip_load4<T, EDGE>(lp, S.inm, S.vin, nxt);
+#pragma unroll
+    for (int h = 1; h <= HL; ++h)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (4 * h - e <= R) o[4 * (HL - h) + e] = __shfl_up_sync(0xffffffffu, o[4 * HL + e], h);
+        if (4 * h + e - 3 <= R) o[4 * (HL + h) + e] = __shfl_down_sync(0xffffffffu, o[4 * HL + e], h);
+      }
+    uint32_t hz[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      hz[c] = 0u;
+#pragma unroll
+      for (int j = 4 * HL + c - R; j <= 4 * HL + c + R; ++j) hz[c] |= o[j];
+    }
+    ring[slot * G::kThreads] = make_uint4(hz[0], hz[1], hz[2], hz[3]);
+    if (S.has_nd) flags[slot * G::kThreads] = f;
+    slot = slot + 1 == P ? 0 : slot + 1;
+    if (i >= 2 * R) {
+      // all slots hold rows of the window
+#pragma unroll
+      for (int s = 0; s < P; ++s) {
+        const uint4 q = ring[s * G::kThreads];
+        hz[0] |= q.x;
+        hz[1] |= q.y;
+        hz[2] |= q.z;
+        hz[3] |= q.w;
+      }
+      uint32_t n[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) n[c] = __popc(hz[c]);
+      const int j = i - 2 * R;
+      if (w) {
+        const uint32_t m = cbuf[j * G::kThreads];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) n[c] += (m >> (8 * c)) & 0xFFu;
+      }
+      if (!last) {
+        cbuf[j * G::kThreads] = n[0] | (n[1] << 8) | (n[2] << 16) | (n[3] << 24);
+      } else {
+        if (S.has_nd) {
+          const uint32_t fc = flags[cslot * G::kThreads];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) n[c] = (fc >> c) & 1u ? 256u : n[c];
+        }
+        if (f64) {
+          uint64_t v[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[c] = out[n[c]];
+          strip_store4<uint64_t>(static_cast<uint64_t*>(a.dst) + orow, v, lane, lo, hi, S.vout, obuf);
+        } else {
+          uint32_t v[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[c] = static_cast<uint32_t>(out[n[c]]);
+          strip_store4<uint32_t>(static_cast<uint32_t*>(a.dst) + orow, v, lane, lo, hi, S.vout,
+                                 reinterpret_cast<uint32_t*>(obuf));
+        }
+      }
+      orow += a.out_pitch;
+    }
+    cslot = cslot + 1 == P ? 0 : cslot + 1;
+  }
+}
+
 template <int R, typename T>
-__global__ void __launch_bounds__(kVyThreads) fs_variety_bits(const FsArgs a, const bool vin, const bool vout) {
+__global__ void __launch_bounds__(VyGeom<R, T>::kThreads) fs_variety_bits(const FsArgs a, const bool vin, const bool vout) {
   using G = VyGeom<R, T>;
   using U = std::make_unsigned_t<T>;
   constexpr int P = G::P, HL = G::HL;
   extern __shared__ __align__(16) unsigned char vy_smem[];
-  __shared__ int wsum[kVyWarps];
+  __shared__ int wsum[G::kWarps];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   uint32_t* lut = reinterpret_cast<uint32_t*>(vy_smem);  // 8-bit: one-hot word of each value in this pass
   uint2* tab = reinterpret_cast<uint2*>(vy_smem);        // 16-bit: (bitmap word, values below it)
-  uint64_t* obuf = reinterpret_cast<uint64_t*>(vy_smem + G::kTab) + 128 * (threadIdx.x >> 5);
-  uint32_t* cbuf = reinterpret_cast<uint32_t*>(vy_smem + G::kTab + G::kBuf);
-  uint4* ring = reinterpret_cast<uint4*>(vy_smem + G::kTab + G::kBuf + G::kCnt);
-  uint32_t* flags = reinterpret_cast<uint32_t*>(ring + P * kVyThreads);
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int64_t xb = static_cast<int64_t>(blockIdx.x) * kVyWarps * G::kCols;  // the block's first output column
-  const int64_t xw = xb + warp * G::kCols - 4 * HL, xs = xw + 4 * lane;
-  const bool active = xw + 4 * HL < a.W;  // warp-uniform
-  const int64_t ys = static_cast<int64_t>(blockIdx.y) * kVyStrip;
-  const int nout = static_cast<int>(a.H - ys < kVyStrip ? a.H - ys : static_cast<int64_t>(kVyStrip));
-  const int nin = nout + 2 * R;
-  const bool has_nd = a.kind == VSR_NODATA_VALUE;
-  const uint32_t ndk = static_cast<U>(static_cast<T>(a.ndv));
+  uint64_t* out = reinterpret_cast<uint64_t*>(vy_smem + G::kTab);
+  uint64_t* obuf = out + kVyOut + 128 * warp;
+  uint4* ring = reinterpret_cast<uint4*>(vy_smem + G::kTab + kVyOut * 8 + G::kBuf) + t;
+  uint32_t* flags = reinterpret_cast<uint32_t*>(ring - t + P * G::kThreads) + t;
+  uint32_t* cbuf = flags + P * G::kThreads;
+  const int64_t xb = static_cast<int64_t>(blockIdx.x) * G::kWarps * G::kCols;  // the block's first output column
   const T* src = static_cast<const T*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride;
-  uint32_t inm = 0;
+  VyStrip S;
+  S.xw = xb + warp * G::kCols - 4 * HL;
+  S.xs = S.xw + 4 * lane;
+  S.ys = static_cast<int64_t>(blockIdx.y) * kVyStrip;
+  S.nout = static_cast<int>(a.H - S.ys < kVyStrip ? a.H - S.ys : static_cast<int64_t>(kVyStrip));
+  S.inm = 0;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) inm |= static_cast<uint32_t>(xs + e >= 0 && xs + e < a.W) << e;
-  auto row_in = [&](int i) { return static_cast<uint64_t>(ys - R + i) < static_cast<uint64_t>(a.H); };
+  for (int e = 0; e < 4; ++e) S.inm |= static_cast<uint32_t>(S.xs + e >= 0 && S.xs + e < a.W) << e;
+  S.vin = vin;
+  S.vout = vout;
+  S.has_nd = a.kind == VSR_NODATA_VALUE;
+  S.ndk = static_cast<U>(static_cast<T>(a.ndv));
+  const bool active = S.xw + 4 * HL < a.W;  // warp-uniform
+  const bool inside = S.xw >= 0 && S.xw + 128 <= a.W;
 
-  // the tile's set of values.  8-bit: a flag word per value (plain stores);
-  // 16-bit: a bitmap, tested before the atomic (most pixels repeat a value)
+  // the tile's set of values
   if (G::kByte) {
-    for (int i = t; i < 256; i += kVyThreads) lut[i] = 0u;
+    for (int i = t; i < 256; i += G::kThreads) lut[i] = 0u;
   } else {
-    for (int i = t; i < 2048; i += kVyThreads) tab[i] = make_uint2(0u, 0u);
+    for (int i = t; i < 2048; i += G::kThreads) tab[i] = make_uint2(0u, 0u);
+  }
+  for (int n = t; n <= 256; n += G::kThreads) {
+    const double v = n == 256 ? a.nd_out : static_cast<double>(n);
+    out[n] = a.out_dtype == VSR_F64 ? static_cast<uint64_t>(__double_as_longlong(v))
+                                    : __float_as_uint(static_cast<float>(v));
   }
   __syncthreads();
-  if (active) {
-    const T* lp = src + (ys - R) * a.pitch + xs;
-#pragma unroll 4
-    for (int i = 0; i < nin; ++i, lp += a.pitch) {
-      if (!row_in(i)) continue;
-      uint32_t e4[4];
-      strip_load4<T>(lp, inm, vin, e4);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (!((inm >> e) & 1u) || (has_nd && e4[e] == ndk)) continue;
-        if (G::kByte) {
-          lut[e4[e]] = 1u;
-        } else {
-          const uint32_t b = 1u << (e4[e] & 31u);
-          if (!(*reinterpret_cast<volatile uint32_t*>(&tab[e4[e] >> 5].x) & b)) atomicOr(&tab[e4[e] >> 5].x, b);
-        }
-      }
-    }
+  if (inside) vy_scan<R, T, false>(a, src, S, lut, tab);
+  else if (active) vy_scan<R, T, true>(a, src, S, lut, tab);
+  __syncthreads();
+  if (t == 0 && S.has_nd) {
+    if (G::kByte) lut[S.ndk] = 0u;
+    else tab[S.ndk >> 5].x &= ~(1u << (S.ndk & 31u));
   }
   __syncthreads();
   // number the values: each thread owns a run of them
-  constexpr int kOwn = (G::kByte ? 256 : 2048) / kVyThreads;  // 8-bit: values; 16-bit: bitmap words
+  constexpr int kOwn = (G::kByte ? 256 : 2048) / G::kThreads;  // 8-bit: values; 16-bit: bitmap words
   uint32_t own[kOwn];
   int cnt = 0;
 #pragma unroll
@@ -246,15 +394,14 @@ __global__ void __launch_bounds__(kVyThreads) fs_variety_bits(const FsArgs a, co
   __syncthreads();
   int base = pre - cnt, total = 0;
 #pragma unroll
-  for (int w = 0; w < kVyWarps; ++w) {
+  for (int w = 0; w < G::kWarps; ++w) {
     base += w < warp ? wsum[w] : 0;
     total += wsum[w];
   }
   if (total > G::kMaxValues) {  // block-uniform
-    __syncthreads();
-    const int64_t x1 = xb + kVyWarps * G::kCols < a.W ? xb + kVyWarps * G::kCols : a.W;
-    for (int64_t y = ys; y < ys + nout; y += kVyTY)
-      for (int64_t x = xb; x < x1; x += kVyTX) variety_pairs<T, R>(a, x, y, x1, vy_smem);
+    const int64_t x1 = xb + G::kWarps * G::kCols < a.W ? xb + G::kWarps * G::kCols : a.W;
+    for (int64_t y = S.ys; y < S.ys + S.nout; y += kVyTY)
+      for (int64_t x = xb; x < x1; x += kVyTX) variety_pairs<T, R, G::kThreads>(a, x, y, x1, vy_smem);
     return;
   }
   if (!G::kByte) {
@@ -266,8 +413,6 @@ __global__ void __launch_bounds__(kVyThreads) fs_variety_bits(const FsArgs a, co
     }
   }
   const int passes = total > 32 ? (total + 31) / 32 : 1;
-  constexpr int lo = 4 * HL;
-  const int hi = static_cast<int>(a.W - xw < 128 - 4 * HL ? a.W - xw : static_cast<int64_t>(128 - 4 * HL));
   for (int w = 0; w < passes; ++w) {
     if (G::kByte) {
       if (w) __syncthreads();  // every thread is done with the last pass's words
@@ -278,102 +423,10 @@ __global__ void __launch_bounds__(kVyThreads) fs_variety_bits(const FsArgs a, co
         b += own[i];
       }
     }
-    __syncthreads();
-    if (!active) continue;
+    if (w == 0 || G::kByte) __syncthreads();
     const bool last = w + 1 == passes;
-    for (int s = 0; s < P; ++s) {
-      ring[s * kVyThreads + t] = make_uint4(0u, 0u, 0u, 0u);
-      flags[s * kVyThreads + t] = 0u;
-    }
-    const T* lp = src + (ys - R) * a.pitch + xs;
-    uint32_t nxt[4];
-    strip_load4<T>(lp, row_in(0) ? inm : 0u, vin, nxt);
-    char* orow = static_cast<char*>(a.dst) +
-                 (static_cast<int64_t>(blockIdx.z) * a.out_band_stride + ys * a.out_pitch + xw) *
-                     (a.out_dtype == VSR_F64 ? 8 : 4);
-    int slot = 0, cslot = P - R;
-#pragma unroll 1
-    for (int i = 0; i < nin; ++i) {
-      uint32_t o[4 * (2 * HL + 1)];
-      const uint32_t in = row_in(i) ? inm : 0u;
-      uint32_t f = 0;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const bool ib = (in >> e) & 1u, nd = ib && has_nd && nxt[e] == ndk;
-        f |= static_cast<uint32_t>(nd) << e;
-        uint32_t word;
-        if (G::kByte) {
-          word = ib ? lut[nxt[e]] : 0u;  // nodata is not in the table
-        } else {
-          const uint2 en = tab[nxt[e] >> 5];
-          const uint32_t rank = en.y + __popc(en.x & ((1u << (nxt[e] & 31u)) - 1u)) - 32u * w;
-          word = ib && !nd && rank < 32u ? 1u << rank : 0u;
-        }
-        o[4 * HL + e] = word;
-      }
-      lp += a.pitch;
-      strip_load4<T>(lp, i + 1 < nin && row_in(i + 1) ? inm : 0u, vin, nxt);
-#pragma unroll
-      for (int h = 1; h <= HL; ++h)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (4 * h - e <= R) o[4 * (HL - h) + e] = __shfl_up_sync(0xffffffffu, o[4 * HL + e], h);
-          if (4 * h + e - 3 <= R) o[4 * (HL + h) + e] = __shfl_down_sync(0xffffffffu, o[4 * HL + e], h);
-        }
-      uint32_t hz[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        hz[c] = 0u;
-#pragma unroll
-        for (int j = 4 * HL + c - R; j <= 4 * HL + c + R; ++j) hz[c] |= o[j];
-      }
-      ring[slot * kVyThreads + t] = make_uint4(hz[0], hz[1], hz[2], hz[3]);
-      flags[slot * kVyThreads + t] = f;
-      slot = slot + 1 == P ? 0 : slot + 1;
-      if (i >= 2 * R) {
-        // the other rows of the window: every other slot
-        int s = slot;
-#pragma unroll
-        for (int k = 0; k < 2 * R; ++k) {
-          const uint4 q = ring[s * kVyThreads + t];
-          s = s + 1 == P ? 0 : s + 1;
-          hz[0] |= q.x;
-          hz[1] |= q.y;
-          hz[2] |= q.z;
-          hz[3] |= q.w;
-        }
-        uint32_t n4 = 0;  // counts, a byte each
-#pragma unroll
-        for (int c = 0; c < 4; ++c) n4 |= static_cast<uint32_t>(__popc(hz[c])) << (8 * c);
-        const int j = i - 2 * R;
-        if (w) n4 += cbuf[j * kVyThreads + t];
-        if (!last) {
-          cbuf[j * kVyThreads + t] = n4;
-        } else {
-          const uint32_t fc = flags[cslot * kVyThreads + t];
-          uint64_t o64[4];
-          uint32_t o32[4];
-          const float ndf = static_cast<float>(a.nd_out);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint32_t n = (n4 >> (8 * c)) & 0xFFu;
-            // a small integer as float by the exponent of 2^23, widened by bits
-            const uint32_t fb = __float_as_uint(__uint_as_float(0x4B000000u | n) - 8388608.0f);
-            const bool nd = (fc >> c) & 1u;
-            o32[c] = nd ? __float_as_uint(ndf) : fb;
-            const uint64_t wide = static_cast<uint64_t>(n ? (fb >> 3) + 0x38000000u : 0u) << 32;
-            o64[c] = nd ? static_cast<uint64_t>(__double_as_longlong(a.nd_out)) : wide;
-          }
-          char* op = orow + static_cast<int64_t>(j) * a.out_pitch * (a.out_dtype == VSR_F64 ? 8 : 4);
-          if (a.out_dtype == VSR_F64)
-            strip_store4<uint64_t>(reinterpret_cast<uint64_t*>(op), o64, lane, lo, hi, vout, obuf);
-          else
-            strip_store4<uint32_t>(reinterpret_cast<uint32_t*>(op), o32, lane, lo, hi, vout,
-                                   reinterpret_cast<uint32_t*>(obuf));
-        }
-      }
-      cslot = cslot + 1 == P ? 0 : cslot + 1;
-    }
+    if (inside) vy_pass<R, T, false>(a, src, S, w, last, lut, tab, out, cbuf, ring, flags, obuf);
+    else if (active) vy_pass<R, T, true>(a, src, S, w, last, lut, tab, out, cbuf, ring, flags, obuf);
   }
 }
 
@@ -382,13 +435,15 @@ int launch_bits(const FsArgs& a, int bands, cudaStream_t st) {
   using G = VyGeom<R, T>;
   const size_t smem = std::max(G::smem(), vy_pairs_smem<VyKey<T>>(R, R));
   auto kern = fs_variety_bits<R, T>;
-  VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  static KernelResidency residency;
+  int per_sm = 0;
+  VSR_CUDA_TRY(residency.get(kern, G::kThreads, smem, &per_sm));
   const bool vin = aligned(a.src, 4 * sizeof(T)) && a.pitch % 4 == 0 && (bands == 1 || a.band_stride % 4 == 0);
   const size_t os = a.out_dtype == VSR_F64 ? 8 : 4;
   const bool vout = aligned(a.dst, 4 * os) && a.out_pitch % 4 == 0 && (bands == 1 || a.out_band_stride % 4 == 0);
-  kern<<<dim3(static_cast<unsigned>((a.W + kVyWarps * G::kCols - 1) / (kVyWarps * G::kCols)),
+  kern<<<dim3(static_cast<unsigned>((a.W + G::kWarps * G::kCols - 1) / (G::kWarps * G::kCols)),
               static_cast<unsigned>((a.H + kVyStrip - 1) / kVyStrip), static_cast<unsigned>(bands)),
-         kVyThreads, smem, st>>>(a, vin, vout);
+         G::kThreads, smem, st>>>(a, vin, vout);
   VSR_CUDA_TRY(cudaGetLastError());
   return VSR_OK;
 }

@@ -135,9 +135,9 @@ int launch_tma_t(const CUtensorMap& map, const HornParams& P, float nd_in, float
   using Tile = TmaTile<TH>;
   const size_t smem = STAGES * Tile::kStride + 1024;
   auto kern = horn_f32_tma<TH, STAGES, THREADS, WANT, NDK, MINB>;
-  VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  static KernelResidency residency;
   int per_sm = 0;
-  VSR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem));
+  VSR_CUDA_TRY(residency.get(kern, THREADS, smem, &per_sm));
   if (per_sm < 1) return fail(VSR_ERR_CUDA, "horn_f32_tma cannot be resident (smem %zu)", smem);
   const int64_t tiles = ((P.width + kTW - 1) / kTW) * ((P.height + TH - 1) / TH) * P.bands;
   const int64_t grid = std::min<int64_t>(tiles, static_cast<int64_t>(sm_count()) * per_sm);

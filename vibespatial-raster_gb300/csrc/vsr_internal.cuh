@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <string>
@@ -42,6 +43,31 @@ uint32_t* device_error_word();  // nullptr (and error set) on failure
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
 int sm_count();  // cached per device
+
+// Dynamic shared memory limit and resident blocks per SM of a kernel, set and
+// asked for once per device (the two calls cost more than a small launch).
+// One instance per kernel, block size and shared-memory size; threads may
+// race to fill it with the same numbers.
+struct KernelResidency {
+  static constexpr int kMaxDevices = 64;
+  std::atomic<int> per_sm[kMaxDevices] = {};
+  template <typename K>
+  cudaError_t get(K kern, int threads, size_t smem, int* out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool keep = dev >= 0 && dev < kMaxDevices;
+    int n = keep ? per_sm[dev].load(std::memory_order_acquire) : 0;
+    if (n == 0) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem);
+      if (e != cudaSuccess) return e;
+      if (keep) per_sm[dev].store(n, std::memory_order_release);
+    }
+    *out = n;
+    return cudaSuccess;
+  }
+};
 
 // Launch-configuration table chosen by the autotuner (vsr_tuning_set).
 int tuning_get(int op);
