@@ -9,11 +9,12 @@
 //   runtime width), one row partial sum per kernel row (for accuracy) and
 //   16-byte broadcast weight loads.  The weight-sum pass runs only on tiles
 //   that touch the border or hold nodata; other tiles use the full sum.
-// * sep_tile     -- the Gaussian as two 1-D passes inside one CTA: the row
-//   pass over the staged tile is held in shared memory and the column pass
-//   reads it.  Numerator and weight sum are both separable, so this equals
-//   the reference's dense k x k normalised correlation with weights
-//   outer(g, g)/sum in real arithmetic, border and nodata handling included.
+// * sep_strip    -- the Gaussian as two 1-D passes inside one CTA: the row
+//   sums are held in shared memory and the column pass reads them.
+//   Numerator and weight sum are both separable, so this equals the
+//   reference's dense k x k normalised correlation with weights outer(g, g) /
+//   sum in real arithmetic, border and nodata handling included.  Kernels of
+//   3 to 17 taps on 8/16-bit and float32 rasters run in gauss_warp.cu.
 // * box_mean     -- focal mean as exact separable sums: int32 for <= 16-bit
 //   integer rasters, float TwoSum pairs for float32, float64 otherwise;
 //   mean = sum / count formed in float64 (reference: Welford in float64,
@@ -312,10 +313,6 @@ int run_conv_direct(const ConvArgs& a, cudaStream_t st, int bands = 1) {
 
 constexpr int kMaxDirectK = 80;
 
-// ------------------------------------------------------------- sep_tile --
-// Separable Gaussian for k <= 33 within a 128 x 32 output tile.
-constexpr int kSTW = 128, kSTH = 32;
-
 struct SepArgs {
   const void* src;
   int dtype;
@@ -328,117 +325,12 @@ struct SepArgs {
   int out_dtype;
   int64_t out_pitch;
   int64_t band_stride, out_band_stride;
+  int seg;  // rows per CTA
 };
 
-inline size_t sep_smem_bytes(int k) {
-  const int SH = kSTH + k - 1, SW = kSTW + k - 1;
-  // staged v*valid and valid, row-pass numerator and denominator, weights
-  return static_cast<size_t>(((2 * SH * padded_width(SW) + 3) & ~3) + 2 * SH * kSTW + ((k + 3) & ~3)) * 4 + 16;
-}
-
-template <int MAXK>
-__global__ void __launch_bounds__(256) sep_tile(const SepArgs a) {
-  extern __shared__ __align__(16) float smem[];
-  const int k = a.k, r = k / 2;
-  const int SH = kSTH + k - 1, SW = kSTW + k - 1, PW = padded_width(SW);
-  float* vz = smem;
-  float* vd = vz + SH * PW;
-  float* rn = vz + ((2 * SH * PW + 3) & ~3);  // SH x kSTW row-pass numerator (16-byte aligned)
-  float* rd = rn + SH * kSTW;
-  float* g = rd + SH * kSTW;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t x0 = static_cast<int64_t>(blockIdx.x) * kSTW;
-  const int64_t y0 = static_cast<int64_t>(blockIdx.y) * kSTH;
-  const void* src = band_src(a.src, a.dtype, a.band_stride);
-  void* dst = band_dst(a.dst, a.out_dtype, a.out_band_stride);
-
-  for (int i = tid; i < k; i += 256) g[i] = a.g32[i];
-  for (int i = tid; i < SH * SW; i += 256) {
-    const int rr = i / SW, c = i - rr * SW;
-    const int64_t gy = y0 + rr - r, gx = x0 + c - r;
-    float v = 0.0f, d = 0.0f;
-    if (gy >= 0 && gy < a.H && gx >= 0 && gx < a.W) {
-      bool ok;
-      const float x = load_elem(src, a.dtype, gy * a.pitch + gx, a.nd, ok);
-      v = x * (ok ? 1.0f : 0.0f);
-      d = ok ? 1.0f : 0.0f;
-    }
-    vz[rr * PW + pos(c)] = v;
-    vd[rr * PW + pos(c)] = d;
-  }
-  __syncthreads();
-
-  // Row pass: each lane 4 adjacent columns of one staged row.
-  for (int rr = warp; rr < SH; rr += 8) {
-    const int c0 = 4 * lane;
-#pragma unroll
-    for (int plane = 0; plane < 2; ++plane) {
-      const float* row = (plane == 0 ? vz : vd) + rr * PW;
-      float V[4 + MAXK - 1];
-#pragma unroll
-      for (int j = 0; j < 4 + MAXK - 1; ++j) V[j] = (j < 4 + k - 1) ? row[pos(c0 + j)] : 0.0f;
-      float acc[4] = {};
-#pragma unroll
-      for (int t = 0; t < MAXK; ++t) {
-        if (t >= k) break;
-        const float w = g[t];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = fmaf(w, V[u + t], acc[u]);
-      }
-      float* o = (plane == 0 ? rn : rd) + rr * kSTW + c0;
-      *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    }
-  }
-  __syncthreads();
-
-  // Column pass: each thread one column, 16 consecutive output rows.
-  constexpr int RY = kSTH / 2;
-  const int c = tid & (kSTW - 1);
-  const int q0 = (tid >> 7) * RY;
-  float num[RY] = {}, den[RY] = {};
-#pragma unroll
-  for (int plane = 0; plane < 2; ++plane) {
-    const float* P = plane == 0 ? rn : rd;
-    float* acc = plane == 0 ? num : den;
-    for (int i = 0; i < RY + k - 1; ++i) {
-      const float v = P[(q0 + i) * kSTW + c];
-#pragma unroll
-      for (int ry = 0; ry < RY; ++ry) {
-        const int t = i - ry;
-        if (t >= 0 && t < k) acc[ry] = fmaf(g[t], v, acc[ry]);
-      }
-    }
-  }
-  const int64_t x = x0 + c;
-  if (x < a.W) {
-#pragma unroll
-    for (int ry = 0; ry < RY; ++ry) {
-      const int64_t y = y0 + q0 + ry;
-      if (y >= a.H) break;
-      const bool centre_ok = vd[(q0 + ry + r) * PW + pos(c + r)] != 0.0f;
-      const double out = (centre_ok && den[ry] > 0.0f) ? static_cast<double>(num[ry] / den[ry]) : a.nd_out;
-      store_out(dst, a.out_dtype, y * a.out_pitch + x, out);
-    }
-  }
-}
-
-template <int MAXK>
-int launch_sep(const SepArgs& a, cudaStream_t st, int bands = 1) {
-  const size_t smem = sep_smem_bytes(a.k);
-  auto kern = sep_tile<MAXK>;
-  VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  dim3 grid(static_cast<unsigned>((a.W + kSTW - 1) / kSTW), static_cast<unsigned>((a.H + kSTH - 1) / kSTH), bands);
-  if (grid.y > 65535u) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the separable Gaussian grid");
-  kern<<<grid, 256, smem, st>>>(a);
-  VSR_CUDA_TRY(cudaGetLastError());
-  return VSR_OK;
-}
-
-constexpr int kMaxSepK = 33;
-
 // ------------------------------------------------------------ sep_strip --
-// Separable Gaussian for large k (> 33, e.g. sigma 8 -> 65 x 65): a CTA walks
-// a 128-column strip down a 512-row segment.  Every input row is reduced
+// Separable Gaussian for what gauss_warp.cu does not take (k >= 19, int32 and
+// float64 rasters): a CTA walks a 128-column strip down a segment of rows.  Every input row is reduced
 // along x once (row pass) into a ring of the last k + 15 row results; every
 // 16 new rows the column pass combines k ring rows into 16 output rows.
 // Numerator (v * valid) and weight sum (valid) travel together as float2
@@ -448,7 +340,7 @@ constexpr int kMaxSepK = 33;
 // shared-memory broadcast.  Work per output pixel: 2k packed FMAs.
 constexpr int kSTW2 = 128;  // strip width
 constexpr int kSBR = 16;    // rows per step
-constexpr int kSSEG = 512;  // rows per CTA segment
+constexpr int kSSEG = 512;  // rows per CTA segment (fewer on small rasters)
 
 __host__ __device__ inline int strip_pos(int i) { return i + (i >> 3); }  // conflict-free 8-wide lane strides
 __host__ __device__ inline int strip_pw(int k) { return strip_pos(kSTW2 + k + 7) + 1; }
@@ -558,8 +450,8 @@ __global__ void __launch_bounds__(256, 2) sep_strip(const SepArgs a) {
   uint32_t* vbits = reinterpret_cast<uint32_t*>(g2 + k8);  // NR x 8 words: staged-column validity bits
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t x0 = static_cast<int64_t>(blockIdx.x) * kSTW2;
-  const int64_t ys = static_cast<int64_t>(blockIdx.y) * kSSEG;
-  const int64_t ye = min(ys + kSSEG, a.H);
+  const int64_t ys = static_cast<int64_t>(blockIdx.y) * a.seg;
+  const int64_t ye = min(ys + a.seg, a.H);
   const void* src = band_src(a.src, a.dtype, a.band_stride);
   void* dst = band_dst(a.dst, a.out_dtype, a.out_band_stride);
   for (int i = tid; i < k8; i += 256) {
@@ -699,7 +591,7 @@ __global__ void __launch_bounds__(256, 2) sep_strip(const SepArgs a) {
   }
 }
 
-int launch_strip(const SepArgs& a, cudaStream_t st, int bands) {
+int launch_strip(SepArgs a, cudaStream_t st, int bands) {
   const size_t smem = strip_smem_bytes(a.k);
   if (smem > 227 * 1024) return fail(VSR_ERR_UNSUPPORTED, "Gaussian kernel %d too large for the strip kernel", a.k);
   // the taps of k in 65..72 (sigma 8 at 4 sigma) are unrolled; other k run-time
@@ -708,7 +600,13 @@ int launch_strip(const SepArgs& a, cudaStream_t st, int bands) {
               : a.dtype == VSR_F32 ? (k9 ? sep_strip<VSR_F32, 9> : sep_strip<VSR_F32, 0>)
                                    : (k9 ? sep_strip<0, 9> : sep_strip<0, 0>);
   VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  dim3 grid(static_cast<unsigned>((a.W + kSTW2 - 1) / kSTW2), static_cast<unsigned>((a.H + kSSEG - 1) / kSSEG), bands);
+  // two CTAs per SM: halve the segments until there are two rounds of them
+  // (a segment reads k - 1 rows more than it writes)
+  const int64_t cols = (a.W + kSTW2 - 1) / kSTW2;
+  a.seg = kSSEG;
+  while (a.seg > 64 && a.seg > 2 * a.k && cols * ((a.H + a.seg - 1) / a.seg) * bands < 4 * static_cast<int64_t>(sm_count()))
+    a.seg /= 2;
+  dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>((a.H + a.seg - 1) / a.seg), bands);
   if (grid.y > 65535u) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the Gaussian grid");
   kern<<<grid, 256, smem, st>>>(a);
   VSR_CUDA_TRY(cudaGetLastError());
@@ -1471,6 +1369,9 @@ int conv_tc_supported(int kh, int kw);
 int run_conv_tc(const void* src, int dtype, int bands, int64_t band_stride, int64_t H, int64_t W, int64_t pitch,
                 const double* weights_host, int kh, int kw, double nodata, int nodata_kind, void* dst, int out_dtype,
                 int64_t out_band_stride, int64_t out_pitch, void* workspace, size_t ws_bytes, cudaStream_t st);
+int run_gauss_warp(const void* src, int dtype, int bands, int64_t band_stride, int64_t H, int64_t W, int64_t pitch,
+                   double sigma, int k, int kind, double ndv, double nd_out, void* dst, int out_dtype,
+                   int64_t out_band_stride, int64_t out_pitch, cudaStream_t st);  // gauss_warp.cu
 int gauss_tc_supported(int dtype, int k);  // gauss_tc.cu
 size_t gauss_tc_workspace(int64_t H, int64_t W, int dtype, int k);
 size_t gauss_tc_workspace_bands(int64_t H, int64_t W, int dtype, int k, int bands);
@@ -1567,9 +1468,10 @@ extern "C" size_t vsr_gaussian_workspace_size(int kernel_size, int precision) {
   return gauss_ws(k);
 }
 
-// VSR_PREC_AUTO takes the split-precision line passes where the separable FP32
-// kernels would use the strip kernel (k > 33) on an 8/16-bit integer raster
-// (exact BF16 hi/lo values) and the caller's workspace holds their planes.
+// VSR_PREC_AUTO takes the split-precision line passes from k = 35 on an
+// 8/16-bit integer raster (exact byte planes) when the caller's workspace holds
+// their sums.
+constexpr int kMaxSepK = 33;
 static bool gauss_tc_auto(int dtype, int64_t height, int64_t width, int k, const void* workspace, size_t bytes) {
   return k > kMaxSepK && gauss_tc_supported(dtype, k) && workspace && aligned(workspace, 256) &&
          bytes >= gauss_tc_workspace(height, width, dtype, k);
@@ -1612,17 +1514,17 @@ static int gaussian_impl(const void* src, int dtype, int bands, int64_t band_str
   if (!workspace || workspace_bytes < need || !aligned(workspace, 256))
     return fail(VSR_ERR_WORKSPACE, "workspace must be 256-byte aligned and >= %zu bytes", need);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const NodataSpec nd = make_nodata(dtype, nodata, nodata_kind);
+  rc = run_gauss_warp(src, dtype, bands, band_stride, height, width, pitch, sigma, k, nd.kind, nd.dv, nodata, dst,
+                      out_dtype, out_band_stride, out_pitch, st);
+  if (rc >= 0) return rc;
   const int k4 = (k + 3) & ~3;
   char* ws = static_cast<char*>(workspace);
   float* g32 = reinterpret_cast<float*>(ws);
   prep_gaussian<<<1, 256, k * sizeof(double), st>>>(k, k4, sigma, g32, nullptr, nullptr);
   VSR_CUDA_TRY(cudaGetLastError());
-  const NodataSpec nd = make_nodata(dtype, nodata, nodata_kind);
   SepArgs a{src, dtype, height, width, pitch, nd, g32, k, nodata, dst, out_dtype, out_pitch, band_stride,
             out_band_stride};
-  if (k <= 8) return launch_sep<8>(a, st, bands);
-  if (k <= 16) return launch_sep<16>(a, st, bands);
-  if (k <= 33) return launch_sep<33>(a, st, bands);
   return launch_strip(a, st, bands);
 }
 
