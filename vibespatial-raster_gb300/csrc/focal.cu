@@ -1369,6 +1369,9 @@ int conv_tc_supported(int kh, int kw);
 int run_conv_tc(const void* src, int dtype, int bands, int64_t band_stride, int64_t H, int64_t W, int64_t pitch,
                 const double* weights_host, int kh, int kw, double nodata, int nodata_kind, void* dst, int out_dtype,
                 int64_t out_band_stride, int64_t out_pitch, void* workspace, size_t ws_bytes, cudaStream_t st);
+int run_conv_warp(const void* src, int dtype, int bands, int64_t band_stride, int64_t H, int64_t W, int64_t pitch,
+                  const double* weights_host, int kh, int kw, int kind, double ndv, double nd_out, void* dst,
+                  int out_dtype, int64_t out_band_stride, int64_t out_pitch, cudaStream_t st);  // conv_warp.cu
 int run_gauss_warp(const void* src, int dtype, int bands, int64_t band_stride, int64_t H, int64_t W, int64_t pitch,
                    double sigma, int k, int kind, double ndv, double nd_out, void* dst, int out_dtype,
                    int64_t out_band_stride, int64_t out_pitch, cudaStream_t st);  // gauss_warp.cu
@@ -1426,6 +1429,10 @@ extern "C" int vsr_convolve_bands(const void* src, int dtype, int bands, int64_t
   if (!workspace || workspace_bytes < need || !aligned(workspace, 256))
     return fail(VSR_ERR_WORKSPACE, "workspace must be 256-byte aligned and >= %zu bytes", need);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const NodataSpec nd = make_nodata(dtype, nodata, nodata_kind);
+  rc = run_conv_warp(src, dtype, bands, band_stride, height, width, pitch, weights_host, kh, kw, nd.kind, nd.dv,
+                     nodata, dst, out_dtype, out_band_stride, out_pitch, st);
+  if (rc >= 0) return rc;
   char* ws = static_cast<char*>(workspace);
   double* w64 = reinterpret_cast<double*>(ws);
   float* w32 = reinterpret_cast<float*>(ws + ((static_cast<size_t>(kh) * kw * 8 + 255) & ~size_t(255)));
@@ -1434,7 +1441,7 @@ extern "C" int vsr_convolve_bands(const void* src, int dtype, int bands, int64_t
   VSR_CUDA_TRY(cudaMemcpyAsync(w64, weights_host, static_cast<size_t>(kh) * kw * 8, cudaMemcpyHostToDevice, st));
   prep_weights<<<1, 256, 0, st>>>(w64, kh, kw, kw4, w32, wsum);
   VSR_CUDA_TRY(cudaGetLastError());
-  ConvArgs a{src, dtype, height, width, pitch, make_nodata(dtype, nodata, nodata_kind), w32, wsum, kh, kw, kw4,
+  ConvArgs a{src, dtype, height, width, pitch, nd, w32, wsum, kh, kw, kw4,
              nodata, dst, out_dtype, out_pitch, bands > 1 ? band_stride : 0, bands > 1 ? out_band_stride : 0};
   return run_conv_direct(a, st, bands);
 }

@@ -9,11 +9,11 @@
 // 2R partial sums of the output rows in flight, and adding a row's term moves
 // each sum one place (acc[j] = g h + acc[j + 1]: an FMA's result may go to
 // another register, so the shift is free).  Column pairs share packed FMAs.
-// No shared memory but for unaligned stores, no barriers.
+// No barriers.
 //
 // The weight sum is a constant while all taps of the strip's last 2R+1 rows
-// are valid (the warp votes once per row); otherwise its partial sums run
-// along, started from the constants when a row with a gap enters.
+// are valid (the warp votes once per row); otherwise the rows' weight sums go
+// through a small ring in shared memory and are added up per output row.
 //
 // The weights are formed in float64 on the host and travel as kernel
 // arguments: FMAs read them from the constant bank, and the call is one
@@ -22,7 +22,6 @@
 // Bound by instruction issue (FMA and shuffles), close to HBM.
 #include <cmath>
 
-#include "df_round.h"
 #include "vsr_internal.cuh"
 #include "warp_strip.cuh"
 
@@ -30,13 +29,7 @@ namespace vsr {
 namespace {
 
 constexpr int kGwMaxR = 8;
-#ifndef GW_STRIP
-#define GW_STRIP 64
-#endif
-#ifndef GW_AHEAD
-#define GW_AHEAD 2
-#endif
-constexpr int kGwAhead = GW_AHEAD;  // rows loaded ahead
+constexpr int kGwDepth = 6;  // rows in shared memory
 
 struct GwArgs {
   const void* src;
@@ -50,21 +43,6 @@ struct GwArgs {
   int strip;
   float g[kGwMaxR + 1];  // g[d]: the weight d from the centre
 };
-
-// A float's float64 bits (exact).
-__device__ __forceinline__ uint64_t widen_bits(float v) {
-  const uint32_t b = __float_as_uint(v);
-  if (!vsr_f32_widen_ok(b)) return static_cast<uint64_t>(__double_as_longlong(static_cast<double>(v)));
-  uint32_t hi, lo;
-  vsr_f32_widen(b, &hi, &lo);
-  return (static_cast<uint64_t>(hi) << 32) | lo;
-}
-
-template <typename T>
-__device__ __forceinline__ float value_of(uint32_t b) {
-  if constexpr (std::is_same<T, float>::value) return __uint_as_float(b);
-  else return static_cast<float>(static_cast<T>(b));
-}
 
 template <int R>
 struct GwGeom {
@@ -109,113 +87,158 @@ __device__ __forceinline__ float2 column_step(float2 acc[2 * R], const float* g,
 template <int R, typename T, typename B>
 __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs a) {
   using G = GwGeom<R>;
+  constexpr int K = G::K;
   constexpr bool kFloat = std::is_same<T, float>::value;
   __shared__ __align__(16) B obuf[128];
+  __shared__ __align__(16) unsigned char rows[RowRing<T, kGwDepth>::kBytes];
+  // while a window holds a gap: the weight sums of its rows and the validity
+  // of the lane's columns (4 bits), each thread reading only its own
+  __shared__ float4 wring[K][32];
+  __shared__ uint32_t oring[K][32];
+  __shared__ float gtab[2 * K];  // the weights twice over, for a ring that starts anywhere
+  auto g_at = [&](int t) { return a.g[t < R ? R - t : t - R]; };
   const int lane = threadIdx.x;
+  for (int t = lane; t < 2 * K; t += 32) gtab[t] = a.g[abs((t < K ? t : t - K) - R)];
   const int64_t xw = static_cast<int64_t>(blockIdx.x) * G::kCols - 4 * G::HL;
   const int64_t xs = xw + 4 * lane, ys = static_cast<int64_t>(blockIdx.y) * a.strip;
   const int nout = static_cast<int>(a.H - ys < a.strip ? a.H - ys : static_cast<int64_t>(a.strip));
   const int nin = nout + 2 * R;
-  uint32_t inm = 0;
+  bool col_out[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) inm |= static_cast<uint32_t>(xs + e >= 0 && xs + e < a.W) << e;
+  for (int e = 0; e < 4; ++e) col_out[e] = xs + e < 0 || xs + e >= a.W;
+  const bool writes = 4 * lane >= 4 * G::HL && 4 * lane < 128 - 4 * G::HL && !col_out[0];
   const T* src = static_cast<const T*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride;
-  const T* lp = src + (ys - R) * a.pitch + xs;
   // input rows [r0, r1) of the strip lie in the raster
   const int r0 = ys < R ? static_cast<int>(R - ys) : 0;
   const int r1 = a.H - (ys - R) < nin ? static_cast<int>(a.H - (ys - R)) : nin;
-  auto load = [&](int i, uint32_t e[4]) {
-    if (i >= r0 && i < r1) strip_load4<T, true>(lp, inm, a.vin, e);
-    lp += a.pitch;
-  };
-  const bool has_nd = a.kind == VSR_NODATA_VALUE, nd_nan = a.kind == VSR_NODATA_NAN;
-  const T ndq = static_cast<T>(a.ndv);
+  const bool nd_nan = a.kind == VSR_NODATA_NAN, nd_val = a.kind == VSR_NODATA_VALUE;
+  const float ndq = nd_val ? static_cast<float>(a.ndv) : __int_as_float(0x7fffffff);  // NaN: equal to nothing
   constexpr int lo = 4 * G::HL;
   const int hi = static_cast<int>(a.W - xw < 128 - 4 * G::HL ? a.W - xw : static_cast<int64_t>(128 - 4 * G::HL));
   B* orow = static_cast<B*>(a.dst) + static_cast<int64_t>(blockIdx.z) * a.out_band_stride + ys * a.out_pitch + xw;
-  // sums of weights of a row and of a window without gaps
-  float rd = a.g[R];
+  // sums of weights of a row (its columns in the raster) and of K such rows
+  float rd[4], wd[4], wr[4];
+  {
+    float f[4];
 #pragma unroll
-  for (int t = 1; t < 2 * R + 1; ++t) rd += a.g[t < R ? R - t : t - R];
-  float wd = a.g[R] * rd;
+    for (int e = 0; e < 4; ++e) f[e] = col_out[e] ? 0.0f : 1.0f;
+    row_sums<R>(f, a.g, rd);
 #pragma unroll
-  for (int t = 1; t < 2 * R + 1; ++t) wd = fmaf(a.g[t < R ? R - t : t - R], rd, wd);
-
-  uint32_t pre[kGwAhead][4];
+    for (int c = 0; c < 4; ++c) {
+      wd[c] = g_at(0) * rd[c];
 #pragma unroll
-  for (int u = 0; u < kGwAhead; ++u) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) pre[u][e] = 0u;
-    load(u, pre[u]);
+      for (int t = 1; t < K; ++t) wd[c] = fmaf(g_at(t), rd[c], wd[c]);
+      wr[c] = strip_recip(wd[c]);
+    }
   }
-  float2 num[2][2 * R], den[2][2 * R];
+  RowRing<T, kGwDepth> in_rows;
+  in_rows.start(rows, src + (ys - R) * a.pitch + xw, a.pitch, xw, a.W, r0, r1, a.vin);
+  float2 num[2][2 * R];
 #pragma unroll
-  for (int j = 0; j < 2 * R; ++j) num[0][j] = num[1][j] = den[0][j] = den[1][j] = make_float2(0.0f, 0.0f);
-  int gaps = 0;     // rows until the last row with a gap leaves the window
-  uint64_t vm = 0;  // validity of the lane's columns, 4 bits per row
-  // not unrolled: two copies of the body overflowed the instruction cache
+  for (int j = 0; j < 2 * R; ++j) num[0][j] = num[1][j] = make_float2(0.0f, 0.0f);
+  int gaps = 0;  // rows until the last row with a gap has left the window
+  int slot = 0;  // ring slot of the row (while gaps > 0)
+  __syncwarp();
+  // not unrolled: more copies of the body outgrow the instruction cache (4
+  // rows per iteration took 263 us where 1 took 192)
 #pragma unroll 1
   for (int i = 0; i < nin; ++i) {
+    uint32_t raw[4];
+    in_rows.take(raw);
     float v[4];
-    uint32_t ok = 0;
+    bool good = true;
+    const bool in = i >= r0 && i < r1;  // a row outside reads as zeros
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      v[e] = value_of<T>(pre[0][e]);
-      bool good;
-      if constexpr (kFloat) good = !(has_nd && v[e] == ndq) && !(nd_nan && v[e] != v[e]);
-      else good = !(has_nd && static_cast<T>(pre[0][e]) == ndq);
-      ok |= good ? 1u << e : 0u;
-#pragma unroll
-      for (int u = 0; u + 1 < kGwAhead; ++u) pre[u][e] = pre[u + 1][e];
+      v[e] = strip_value<T>(raw[e]);
+      good = good && ((v[e] != ndq && !(kFloat && nd_nan && v[e] != v[e])) || col_out[e]);
     }
-    ok &= inm;
-    const bool in = i >= r0 && i < r1;
-    if (!in) ok = 0u;
-    load(i + kGwAhead, pre[kGwAhead - 1]);
-    vm = (vm << 4) | ok;
-    const bool gap = !__all_sync(0xffffffffu, ok == 0xFu);
+    const bool gap = !__all_sync(0xffffffffu, good || !in);
+    uint32_t ok = 0xFu;
     if (gap) {
-      // v * valid, as the reference masks: a NaN stays NaN under a zero
+      ok = 0u;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = in ? v[e] * ((ok >> e) & 1u ? 1.0f : 0.0f) : 0.0f;
-      if (gaps == 0) {  // rows so far had none: acc[j] holds the constant terms t = 0 .. 2R - 1 - j
-        float s = a.g[R] * rd;
-#pragma unroll
-        for (int j = 2 * R - 1; j >= 0; --j) {
-          den[0][j] = den[1][j] = make_float2(s, s);
-          const int t = 2 * R - j;
-          s = fmaf(a.g[t < R ? R - t : t - R], rd, s);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const bool o = !col_out[e] && v[e] != ndq && !(kFloat && nd_nan && v[e] != v[e]);
+        ok |= o ? 1u << e : 0u;
+        v[e] *= o ? 1.0f : 0.0f;  // as the reference masks: a NaN stays NaN under a zero
       }
-      gaps = 2 * R + 1;
+      if (gaps == 0) {  // the rows before had none
+        for (int t = 1; t < K; ++t) {
+          const bool ti = i - K + t >= r0 && i - K + t < r1;
+          wring[t][lane] = ti ? make_float4(rd[0], rd[1], rd[2], rd[3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          oring[t][lane] = 0xFu;
+        }
+        slot = 0;
+      }
+      gaps = K;
     }
     float h[4];
     row_sums<R>(v, a.g, h);
     const float2 o0 = column_step<R>(num[0], a.g, make_float2(h[0], h[1]));
     const float2 o1 = column_step<R>(num[1], a.g, make_float2(h[2], h[3]));
-    float2 d0 = make_float2(wd, wd), d1 = d0;
+    const float n4[4] = {o0.x, o0.y, o1.x, o1.y};
+    uint32_t cm = 0xFu;  // validity of the output row's columns
+    float w4[4], r4[4];
+    bool whole = false;
     if (gaps) {
       --gaps;
-      float w[4] = {rd, rd, rd, rd};
+      float w[4] = {rd[0], rd[1], rd[2], rd[3]};
       if (gap) {
         float f[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) f[e] = (ok >> e) & 1u ? 1.0f : 0.0f;
         row_sums<R>(f, a.g, w);
       }
-      d0 = column_step<R>(den[0], a.g, make_float2(w[0], w[1]));
-      d1 = column_step<R>(den[1], a.g, make_float2(w[2], w[3]));
+      wring[slot][lane] = in ? make_float4(w[0], w[1], w[2], w[3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      oring[slot][lane] = ok;
+      slot = slot + 1 == K ? 0 : slot + 1;
+      // slot s holds the row of weight (s - slot) mod K
+      float2 d0 = make_float2(0.0f, 0.0f), d1 = d0;
+      const float* gs = gtab + K - slot;
+#pragma unroll
+      for (int s = 0; s < K; ++s) {
+        const float4 x = wring[s][lane];
+        const float2 gt = make_float2(gs[s], gs[s]);
+        d0 = __ffma2_rn(gt, make_float2(x.x, x.y), d0);
+        d1 = __ffma2_rn(gt, make_float2(x.z, x.w), d1);
+      }
+      const int cs = slot + R;
+      cm = oring[cs >= K ? cs - K : cs][lane];
+      w4[0] = d0.x;
+      w4[1] = d0.y;
+      w4[2] = d1.x;
+      w4[3] = d1.y;
+    } else if (i - 2 * R < r0 || i >= r1) {  // rows outside: only those inside weigh
+      float cs = 0.0f;
+#pragma unroll
+      for (int t = 0; t < K; ++t) cs += i - 2 * R + t >= r0 && i - 2 * R + t < r1 ? g_at(t) : 0.0f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) w4[c] = rd[c] * cs;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) w4[c] = wd[c];
+      whole = true;
     }
     if (i >= 2 * R) {
-      const uint32_t cm = static_cast<uint32_t>(vm >> (4 * R));
-      const float n4[4] = {o0.x, o0.y, o1.x, o1.y}, w4[4] = {d0.x, d0.y, d1.x, d1.y};
       B b[4];
+      bool bad = false;
+      float q[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        r4[c] = whole ? wr[c] : strip_recip(w4[c]);
+        bad |= !(w4[c] > 1.0e-30f);
+        q[c] = strip_quot(n4[c], w4[c], r4[c], bad);
+      }
+      if (bad && writes) {  // a lane that writes nothing may hold anything
+#pragma unroll
+        for (int c = 0; c < 4; ++c) q[c] = n4[c] / w4[c];
+      }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const bool nd = !((cm >> c) & 1u) || !(w4[c] > 0.0f);
-        const float q = n4[c] / w4[c];
-        if constexpr (sizeof(B) == 8) b[c] = nd ? static_cast<B>(__double_as_longlong(a.nd_out)) : widen_bits(q);
-        else b[c] = __float_as_uint(nd ? static_cast<float>(a.nd_out) : q);
+        if constexpr (sizeof(B) == 8) b[c] = nd ? static_cast<B>(__double_as_longlong(a.nd_out)) : widen_bits(q[c]);
+        else b[c] = __float_as_uint(nd ? static_cast<float>(a.nd_out) : q[c]);
       }
       strip_store4<B>(orow, b, lane, lo, hi, a.vout, obuf);
       orow += a.out_pitch;
@@ -226,7 +249,11 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
 template <int R, typename T>
 int launch_gw(GwArgs& a, int bands, bool f64, cudaStream_t st) {
   const int64_t gx = (a.W + GwGeom<R>::kCols - 1) / GwGeom<R>::kCols;
-  a.strip = GW_STRIP;
+  // rows per strip: the most that gives every SM 32 warps, two rounds of what
+  // fits (2R rows of a strip are read again by the next; 900 x 6000, 13 taps: 77 us at
+  // 64 rows, 54 us at 32)
+  a.strip = 64;
+  while (a.strip > 16 && gx * ((a.H + a.strip - 1) / a.strip) * bands < 32 * static_cast<int64_t>(sm_count())) a.strip /= 2;
   const int64_t gy = (a.H + a.strip - 1) / a.strip;
   if (gy > 65535) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the separable Gaussian grid");
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(bands));
