@@ -135,14 +135,14 @@ __global__ void __launch_bounds__(32) conv_warp(const __grid_constant__ CwArgs a
     for (int e = 0; e < 4; ++e) {
       const float v = strip_value<T>(raw[e]);
       w[C0 + e] = v;
-      good = good && ((v != ndq && !(kFloat && nd_nan && v != v)) || col_out[e]);
+      good &= ((v != ndq) & !(kFloat & nd_nan & (v != v))) | col_out[e];
     }
     if (!__all_sync(0xffffffffu, good && in)) {
       uint32_t ok = 0u;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float v = w[C0 + e];
-        const bool o = in && !col_out[e] && v != ndq && !(kFloat && nd_nan && v != v);
+        const bool o = in & !col_out[e] & (v != ndq) & !(kFloat & nd_nan & (v != v));
         ok |= o ? 1u << e : 0u;
         w[C0 + e] = v * (o ? 1.0f : 0.0f);  // as the reference masks: a NaN stays NaN under a zero
       }
@@ -206,11 +206,16 @@ __global__ void __launch_bounds__(32) conv_warp(const __grid_constant__ CwArgs a
         for (int c = 0; c < 4; ++c) q[c] = done[c] / d[c];
       }
       B b[4];
+      bool nd[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const bool nd = !((cm >> c) & 1u) || !(d[c] > 0.0f);
-        if constexpr (sizeof(B) == 8) b[c] = nd ? static_cast<B>(__double_as_longlong(a.nd_out)) : widen_bits(q[c]);
-        else b[c] = __float_as_uint(nd ? static_cast<float>(a.nd_out) : q[c]);
+      for (int c = 0; c < 4; ++c) nd[c] = !((cm >> c) & 1u) | !(d[c] > 0.0f);
+      if constexpr (sizeof(B) == 8) {
+        widen4(q, b);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = nd[c] ? static_cast<B>(__double_as_longlong(a.nd_out)) : b[c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = __float_as_uint(nd[c] ? static_cast<float>(a.nd_out) : q[c]);
       }
       strip_store4<B>(orow, b, lane, lo, hi, a.vout, obuf);
       orow += a.out_pitch;
@@ -226,7 +231,8 @@ int launch_cw(CwArgs& a, int bands, bool f64, cudaStream_t st) {
   a.strip = 64;
   while (a.strip > 16 && gx * ((a.H + a.strip - 1) / a.strip) * bands < 32 * static_cast<int64_t>(sm_count())) a.strip /= 2;
   const int64_t gy = (a.H + a.strip - 1) / a.strip;
-  if (gy > 65535) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the direct convolution grid");
+  if ((a.H + 31) / 32 > 65535 || gy > 65535)
+    return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the direct convolution grid");
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(bands));
   if (f64) conv_warp<K, T, uint64_t><<<grid, 32, 0, st>>>(a);
   else conv_warp<K, T, uint32_t><<<grid, 32, 0, st>>>(a);

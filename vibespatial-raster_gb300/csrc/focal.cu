@@ -1525,6 +1525,8 @@ static int gaussian_impl(const void* src, int dtype, int bands, int64_t band_str
   rc = run_gauss_warp(src, dtype, bands, band_stride, height, width, pitch, sigma, k, nd.kind, nd.dv, nodata, dst,
                       out_dtype, out_band_stride, out_pitch, st);
   if (rc >= 0) return rc;
+  if (k <= kMaxSepK && (height + 31) / 32 > 65535)
+    return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the separable Gaussian grid");
   const int k4 = (k + 3) & ~3;
   char* ws = static_cast<char*>(workspace);
   float* g32 = reinterpret_cast<float*>(ws);

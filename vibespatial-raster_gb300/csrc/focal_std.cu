@@ -176,13 +176,13 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
         bool nd, ok;
         if constexpr (kFloat) {
           const bool eq = v == S.ndq;
-          ok = !eq && v == v;
+          ok = !eq & (v == v);
           nd = nd_nan ? v != v : eq;
         } else {
-          nd = has_nd && v == ndv;
+          nd = has_nd & (v == ndv);
           ok = !nd;
         }
-        if (EDGE) ok = ok && ((inm >> e) & 1u);  // nd outside the raster: never a centre that is written
+        if (EDGE) ok = ok & ((inm >> e) & 1u);  // nd outside the raster: never a centre that is written
         f |= ok ? 1u << (8 * e) : 0u;
         f |= nd ? 2u << (8 * e) : 0u;
         if constexpr (!kFloat) {
@@ -340,8 +340,8 @@ __device__ __forceinline__ void scan_range(const FsArgs& a, const SdStrip& S, bo
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float v = __uint_as_float(raw[e]);
-      bool ok = v != S.ndq && v == v;
-      if (EDGE) ok = ok && ((inm >> e) & 1u);
+      bool ok = (v != S.ndq) & (v == v);
+      if (EDGE) ok = ok & ((inm >> e) & 1u);
       amin = min(amin, ok ? (raw[e] & 0x7fffffffu) - 1u : 0xFFFFFFFFu);
       vmin = fminf(vmin, ok ? v : __int_as_float(0x7f800000));
       vmax = fmaxf(vmax, ok ? v : __int_as_float(0xff800000));

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       v[e] = strip_value<T>(raw[e]);
-      good = good && ((v[e] != ndq && !(kFloat && nd_nan && v[e] != v[e])) || col_out[e]);
+      good &= ((v[e] != ndq) & !(kFloat & nd_nan & (v[e] != v[e]))) | col_out[e];
     }
     const bool gap = !__all_sync(0xffffffffu, good || !in);
     uint32_t ok = 0xFu;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
       ok = 0u;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const bool o = !col_out[e] && v[e] != ndq && !(kFloat && nd_nan && v[e] != v[e]);
+        const bool o = !col_out[e] & (v[e] != ndq) & !(kFloat & nd_nan & (v[e] != v[e]));
         ok |= o ? 1u << e : 0u;
         v[e] *= o ? 1.0f : 0.0f;  // as the reference masks: a NaN stays NaN under a zero
       }
@@ -234,11 +234,16 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
 #pragma unroll
         for (int c = 0; c < 4; ++c) q[c] = n4[c] / w4[c];
       }
+      bool nd[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const bool nd = !((cm >> c) & 1u) || !(w4[c] > 0.0f);
-        if constexpr (sizeof(B) == 8) b[c] = nd ? static_cast<B>(__double_as_longlong(a.nd_out)) : widen_bits(q[c]);
-        else b[c] = __float_as_uint(nd ? static_cast<float>(a.nd_out) : q[c]);
+      for (int c = 0; c < 4; ++c) nd[c] = !((cm >> c) & 1u) | !(w4[c] > 0.0f);
+      if constexpr (sizeof(B) == 8) {
+        widen4(q, b);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = nd[c] ? static_cast<B>(__double_as_longlong(a.nd_out)) : b[c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = __float_as_uint(nd[c] ? static_cast<float>(a.nd_out) : q[c]);
       }
       strip_store4<B>(orow, b, lane, lo, hi, a.vout, obuf);
       orow += a.out_pitch;
@@ -255,7 +260,8 @@ int launch_gw(GwArgs& a, int bands, bool f64, cudaStream_t st) {
   a.strip = 64;
   while (a.strip > 16 && gx * ((a.H + a.strip - 1) / a.strip) * bands < 32 * static_cast<int64_t>(sm_count())) a.strip /= 2;
   const int64_t gy = (a.H + a.strip - 1) / a.strip;
-  if (gy > 65535) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the separable Gaussian grid");
+  if ((a.H + 31) / 32 > 65535 || gy > 65535)
+    return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the separable Gaussian grid");
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(bands));
   if (f64) gauss_warp<R, T, uint64_t><<<grid, 32, 0, st>>>(a);
   else gauss_warp<R, T, uint32_t><<<grid, 32, 0, st>>>(a);

@@ -5,11 +5,12 @@
 // down-cast passes of their launch glue (algebra.py:2257-2383, 2632-2775).
 // The arithmetic is in horn_common.cuh.
 //
-// Two kernels:
+// Three kernels:
 //  * horn_f32_tma  -- float32 rasters with 16-byte aligned rows
 //    (horn_tma.cuh; instantiated in horn_tma_all.cu / horn_tma_sub.cu).
-//  * horn_generic  -- every other dtype / alignment: one thread per pixel,
-//    clamped loads through L1.
+//  * horn_strip    -- 8/16-bit rasters and other float32 ones (horn_strip.cu).
+//  * horn_generic  -- int32 and float64: one thread per pixel, clamped loads
+//    through L1.
 #include <type_traits>
 
 #include "horn_common.cuh"
@@ -20,6 +21,8 @@ namespace horn {
 template <int WANT>
 int launch_tma_want(int cfg, const CUtensorMap& map, const HornParams& P, float nd_in, float* slope, float* aspect,
                     uint8_t* hs, uint32_t* err, cudaStream_t st);
+int run_horn_strip(int dtype, const void* src, const HornParams& P, double ndv, void* slope, void* aspect, bool f64,
+                   uint8_t* hs, cudaStream_t st);  // horn_strip.cu
 
 namespace {
 
@@ -40,11 +43,6 @@ __device__ __forceinline__ PixelOut horn_pixel(float gx, float gy, const HornPar
   return o;
 }
 
-template <typename T>
-struct DiffType { using type = float; };
-template <> struct DiffType<double> { using type = double; };
-template <> struct DiffType<int32_t> { using type = double; };
-
 template <typename O> __device__ __forceinline__ O nd_out(const HornParams& P);
 template <> __device__ __forceinline__ float nd_out<float>(const HornParams& P) { return P.nd_out_f; }
 template <> __device__ __forceinline__ double nd_out<double>(const HornParams& P) { return P.nd_out_d; }
@@ -53,7 +51,7 @@ template <typename T, typename O>
 __global__ void __launch_bounds__(256) horn_generic(const T* __restrict__ src, const HornParams P,
                                                     const NodataTest<T> nd, O* __restrict__ slope,
                                                     O* __restrict__ aspect, uint8_t* __restrict__ hs) {
-  using D = typename DiffType<T>::type;
+  using D = double;
   const int64_t x = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
   const int64_t y = static_cast<int64_t>(blockIdx.y) * 8 + threadIdx.y;
   if (x >= P.width || y >= P.height) return;
@@ -79,13 +77,8 @@ __global__ void __launch_bounds__(256) horn_generic(const T* __restrict__ src, c
     }
   }
   float gx, gy;
-  if constexpr (std::is_same<T, float>::value) {  // float differences may round (see grad_exact)
-    gx = grad_exact(v[0][0], v[0][2], v[1][0], v[1][2], v[2][0], v[2][2]);
-    gy = grad_exact(v[0][0], v[2][0], v[0][1], v[2][1], v[0][2], v[2][2]);
-  } else {  // exact: small integers in float, wider types in double
-    gx = static_cast<float>((v[0][2] - v[0][0]) + D(2) * (v[1][2] - v[1][0]) + (v[2][2] - v[2][0]));
-    gy = static_cast<float>((v[2][0] - v[0][0]) + D(2) * (v[2][1] - v[0][1]) + (v[2][2] - v[0][2]));
-  }
+  gx = static_cast<float>((v[0][2] - v[0][0]) + D(2) * (v[1][2] - v[1][0]) + (v[2][2] - v[2][0]));
+  gy = static_cast<float>((v[2][0] - v[0][0]) + D(2) * (v[2][1] - v[0][1]) + (v[2][2] - v[0][2]));
   const PixelOut o = horn_pixel(gx, gy, P, slope != nullptr, aspect != nullptr, hs != nullptr);
   const bool sa_nd = rule.sa_any && (rule.sa_center ? ctr : dil);
   if (slope) slope[y * P.out_pitch + x] = sa_nd ? nd_out<O>(P) : static_cast<O>(o.slope);
@@ -111,11 +104,7 @@ template <typename O>
 int dispatch_generic(int dtype, const void* src, const HornParams& P, double ndv, void* slope,
                      void* aspect, uint8_t* hs, cudaStream_t st) {
   switch (dtype) {
-    case VSR_F32: return launch_generic<float, O>(src, P, ndv, slope, aspect, hs, st);
     case VSR_F64: return launch_generic<double, O>(src, P, ndv, slope, aspect, hs, st);
-    case VSR_U8: return launch_generic<uint8_t, O>(src, P, ndv, slope, aspect, hs, st);
-    case VSR_I16: return launch_generic<int16_t, O>(src, P, ndv, slope, aspect, hs, st);
-    case VSR_U16: return launch_generic<uint16_t, O>(src, P, ndv, slope, aspect, hs, st);
     case VSR_I32: return launch_generic<int32_t, O>(src, P, ndv, slope, aspect, hs, st);
     default: return fail(VSR_ERR_INVALID_ARG, "unsupported dtype %d", dtype);
   }
@@ -230,6 +219,9 @@ extern "C" int vsr_horn_fused_bands(const void* dem, int dtype, int bands, int64
   if (tma_ok)
     return launch_tma_config(tuning_get(VSR_OP_HORN), dem, P, static_cast<float>(ndv),
                              static_cast<float*>(slope), static_cast<float*>(aspect), hillshade, st);
+  const int rc = run_horn_strip(dtype, dem, P, ndv, slope, aspect, (slope || aspect) && out_dtype == VSR_F64,
+                                hillshade, st);
+  if (rc >= 0) return rc;
   if ((slope || aspect) && out_dtype == VSR_F64)
     return dispatch_generic<double>(dtype, dem, P, ndv, slope, aspect, hillshade, st);
   return dispatch_generic<float>(dtype, dem, P, ndv, slope, aspect, hillshade, st);

@@ -36,35 +36,37 @@ VSR_TF_FN int vsr_tf_clz32(uint32_t v) {  // v != 0
 #endif
 }
 
+VSR_TF_FN uint32_t vsr_tf_shl(uint32_t hi, uint32_t lo, int z) {  // high word of (hi, lo) << z, 0 <= z < 32
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_l(lo, hi, z);
+#else
+  return z ? (hi << z) | (lo >> (32 - z)) : hi;
+#endif
+}
+
 // float64 bits of -(a kx + b ky) 2^u; |a|, |b| < 2^29 and a normal result.
+// Without branches: lanes differ in sign and length.  A negative value is
+// taken as its ones' complement, one unit of 2^-s (2^-59 of a factor) off.
 VSR_TF_FN uint64_t vsr_curv_bits(int32_t a, int32_t b, const vsr_curv_k* k, int u) {
-  const int64_t sl = (int64_t)a * k->xl + (int64_t)b * k->yl;  // < 2^61
-  const int64_t sh = (int64_t)a * k->xh + (int64_t)b * k->yh;  // < 2^59
-  int64_t vh = sh + (sl >> 31);
-  uint32_t vl = (uint32_t)sl & 0x7fffffffu;  // value = vh 2^31 + vl
-  const uint32_t neg = vh < 0;
-  if (neg) {
-    vh = ~vh + (vl == 0u);
-    vl = (0u - vl) & 0x7fffffffu;
-  }
-  uint64_t m = (uint64_t)vh, r = (uint64_t)vl << 33;  // m.r, r the fraction bits left-aligned
-  int e = 63 + 31;
-  if (m == 0u) {
-    m = r;
-    r = 0u;
-    e -= 64;
-    if (m == 0u) return 0u;
-  }
-  if ((uint32_t)(m >> 32) == 0u) {
-    m = (m << 32) | (r >> 32);
-    r <<= 32;
-    e -= 32;
-  }
-  const int z = vsr_tf_clz32((uint32_t)(m >> 32));
-  m = z ? (m << z) | (r >> (64 - z)) : m;
-  const uint64_t mant = (m >> 11) + ((m >> 10) & 1u);
-  const uint32_t be = (uint32_t)(e - z + u - k->s + 1023 - 1);
-  return ((uint64_t)((neg ^ 1u) << 31 | be << 20) << 32) + mant;
+  const int64_t sl = (int64_t)a * k->xl + (int64_t)b * k->yl;                // < 2^61
+  const int64_t vh = (int64_t)a * k->xh + (int64_t)b * k->yh + (sl >> 31);   // < 2^60
+  const uint32_t neg = (uint32_t)(int32_t)(vh >> 63);  // all ones when negative
+  // |value| = (x0, x1, x2 / 2^32) 2^31
+  uint32_t x0 = (uint32_t)((uint64_t)vh >> 32) ^ neg, x1 = (uint32_t)vh ^ neg, x2 = ((uint32_t)sl ^ neg) << 1;
+  int e = 63 + 31 + 1023 - 1 + u - k->s;
+  const int s1 = x0 == 0u;
+  x0 = s1 ? x1 : x0;
+  x1 = s1 ? x2 : x1;
+  x2 = s1 ? 0u : x2;
+  const int s2 = x0 == 0u;
+  x0 = s2 ? x1 : x0;
+  x1 = s2 ? x2 : x1;
+  e -= (s1 ? 32 : 0) + (s2 ? 32 : 0);
+  const int z = vsr_tf_clz32(x0 | 1u);
+  const uint32_t f0 = vsr_tf_shl(x0, x1, z), f1 = vsr_tf_shl(x1, s2 ? 0u : x2, z);
+  const uint64_t m = ((uint64_t)(f0 >> 11) << 32 | vsr_tf_shl(f0, f1, 21)) + ((f1 >> 10) & 1u);
+  const uint64_t r = m + ((uint64_t)((uint32_t)(e - z) << 20 | (~neg & 0x80000000u)) << 32);
+  return x0 ? r : 0u;
 }
 
 #endif

@@ -33,13 +33,13 @@ constexpr int kTsDepth = 6;  // rows in shared memory
 // way differences stay below 2^28 and the sums of eight below 2^31.
 constexpr uint32_t kTsSpan = 4, kTsSpanPos = 5;
 
-// float64 bits of s 2^e: s + 2^31 as the low word of 2^52 + ., one FP64 subtraction.
-__device__ __forceinline__ uint64_t scaled_bits(int32_t s, int e) {
+// float64 bits of s 2^e, e20 = e 2^20: s + 2^31 as the low word of 2^52 + .,
+// one FP64 subtraction.
+__device__ __forceinline__ uint64_t scaled_bits(int32_t s, uint32_t e20) {
   const double d = __hiloint2double(0x43300000, s ^ static_cast<int32_t>(0x80000000u)) -
                    (4503599627370496.0 + 2147483648.0);
-  uint64_t b = static_cast<uint64_t>(__double_as_longlong(d));
-  if (s) b += static_cast<uint64_t>(static_cast<uint32_t>(e) << 20) << 32;
-  return b;
+  return static_cast<uint64_t>(__double_as_longlong(
+      __hiloint2double(__double2hiint(d) + static_cast<int32_t>(s ? e20 : 0u), __double2loint(d))));
 }
 
 template <typename B>
@@ -83,8 +83,11 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
     writes |= static_cast<uint32_t>(p >= 1 && p <= kTsCols && xw + p < P.W) << j;
     side |= static_cast<uint32_t>(xw + p == 0 || xw + p == P.W - 1) << j;
   }
+  const bool edge = xw < 0 || xw + 128 >= P.W;  // the strip has a border column
   const bool nd_nan = P.nd_kind == VSR_NODATA_NAN, nd_any = P.nd_kind != VSR_NODATA_NONE;
   const T ndv = static_cast<T>(P.nd_in);
+  // a float32 DEM's nodata value, or NaN (equal to nothing)
+  const float ndq = P.nd_kind == VSR_NODATA_VALUE ? static_cast<float>(P.nd_in) : __int_as_float(0x7fffffff);
   const int64_t o0 = static_cast<int64_t>(blockIdx.z) * P.out_band_stride + ys * P.out_pitch + xw + lane;
   B* tri = P.tri ? static_cast<B*>(P.tri) + o0 : nullptr;
   B* tpi = P.tpi ? static_cast<B*>(P.tpi) + o0 : nullptr;
@@ -109,9 +112,11 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       v[j] = row[32 * j];
-      nd[j] = nd_any && (nd_nan ? v[j] != v[j] : v[j] == ndv);
       if constexpr (kFloat) {
-        fits = fits && (nd[j] || v[j] == 0.0f || (__float_as_uint(v[j]) & signs) - (e0 << 23) < span << 23);
+        nd[j] = (v[j] == ndq) | (nd_nan & (v[j] != v[j]));
+        fits &= nd[j] | (v[j] == 0.0f) | ((__float_as_uint(v[j]) & signs) - (e0 << 23) < span << 23);
+      } else {
+        nd[j] = nd_any & (v[j] == ndv);
       }
     }
     int32_t bl[4], bc[4], br[4];
@@ -189,41 +194,47 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
     }
     if (i >= 2) {
       const int64_t y = ys + i - 2;
-      uint32_t flag = y == 0 || y == P.H - 1 ? 0xFu : side;  // bit j: nodata
-#pragma unroll
-      for (int j = 0; j < 4; ++j) flag |= ((dt[j] | dm[j] | db[j]) >> lane & 1u) << j;
       if (shared && P.ck.ok) {
         const int u = kFloat ? static_cast<int>(e0) - 150 : 0;
+        const uint32_t e20 = static_cast<uint32_t>(u - 3) << 20;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int32_t c = mc[j];
-          const bool w = writes >> j & 1u, nd1 = flag >> j & 1u;
+          const bool w = writes >> j & 1u;
           if (tri) {
             const int32_t s = (abs(tl[j] - c) + abs(tc[j] - c)) + (abs(tr[j] - c) + abs(ml[j] - c)) +
                               (abs(mr[j] - c) + abs(bl[j] - c)) + (abs(bc[j] - c) + abs(br[j] - c));
-            const B b = out_bits<B>(scaled_bits(s, u - 3));
-            if (w) __stcs(tri + 32 * j, nd1 ? ndb : b);
+            const B b = out_bits<B>(scaled_bits(s, e20));
+            if (w) tri[32 * j] = b;
           }
           if (tpi) {
             const int32_t s = 8 * c - ((tl[j] + tc[j] + tr[j]) + (ml[j] + mr[j]) + (bl[j] + bc[j] + br[j]));
-            const B b = out_bits<B>(scaled_bits(s, u - 3));
-            if (w) __stcs(tpi + 32 * j, nd1 ? ndb : b);
+            const B b = out_bits<B>(scaled_bits(s, e20));
+            if (w) tpi[32 * j] = b;
           }
           if (curv) {
             const B b = out_bits<B>(vsr_curv_bits(ml[j] + mr[j] - 2 * c, tc[j] + bc[j] - 2 * c, &P.ck, u));
-            if (w) __stcs(curv + 32 * j, nd1 ? ndb : b);
+            if (w) curv[32 * j] = b;
           }
         }
       } else {
 #pragma unroll 1
+        for (int j = 0; j < 4; ++j)
+          if (writes >> j & 1u) slow_pixel<T>(src, P, xw + 32 * j + lane, y);
+      }
+      // borders and windows that touch nodata, over what was just written
+      const bool border = y == 0 || y == P.H - 1;
+      uint32_t any = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) any |= dt[j] | dm[j] | db[j];
+      if (any || border || edge) {
+#pragma unroll
         for (int j = 0; j < 4; ++j) {
-          if (!(writes >> j & 1u)) continue;
-          if (flag >> j & 1u) {
+          const bool f = border || (side >> j & 1u) || ((dt[j] | dm[j] | db[j]) >> lane & 1u);
+          if (f && (writes >> j & 1u)) {
             if (tri) tri[32 * j] = ndb;
             if (tpi) tpi[32 * j] = ndb;
             if (curv) curv[32 * j] = ndb;
-          } else {
-            slow_pixel<T>(src, P, xw + 32 * j + lane, y);
           }
         }
       }
@@ -255,7 +266,8 @@ int launch_ts(const void* dem, const DerivParams& P, int bands, cudaStream_t st)
   int strip = 64;
   while (strip > 8 && gx * ((P.H + strip - 1) / strip) * bands < 32 * static_cast<int64_t>(sm_count())) strip /= 2;
   const int64_t gy = (P.H + strip - 1) / strip;
-  if (gy > 65535) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the terrain-derivative grid");
+  if ((P.H + 7) / 8 > 65535 || gy > 65535)
+    return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the terrain-derivative grid");
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(bands));
   if (P.out_dtype == VSR_F64)
     terrain_strip<T, unsigned long long><<<grid, 32, 0, st>>>(static_cast<const T*>(dem), P, strip);
