@@ -37,13 +37,14 @@ import numpy as np
 from vsr_gb300 import _lib
 from vsr_gb300.buffers import (
     OwnedRasterArray,
-    RasterDiagnosticEvent,
     RasterDiagnosticKind,
+    diagnostic_event,
     from_device,
     torch_dtype,
 )
 from vsr_gb300.residency import Residency
 
+_F64 = np.dtype(np.float64)
 _GPU_ONLY = (
     "vsr_gb300 runs focal operations on the GPU only; use the reference package "
     "for its CPU path (use_gpu=False)"
@@ -68,14 +69,16 @@ def _should_use_gpu(raster: OwnedRasterArray, threshold: int = 10_000) -> bool:
 def _require_gpu(use_gpu) -> None:
     if use_gpu is False:
         raise NotImplementedError(_GPU_ONLY)
-    torch = _torch()
-    if not torch.cuda.is_available():
+    cuda = _torch().cuda
+    if not (cuda.is_initialized() or cuda.is_available()):
         raise RuntimeError("vsr_gb300 needs a CUDA device (GB300, sm_103a)")
     _lib.load()
 
 
 def _stream_handle():
-    return _torch().cuda.current_stream().cuda_stream
+    """The current device's current stream as a raw handle (no Stream object)."""
+    torch = _torch()
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def cellsize(affine) -> tuple[float, float]:
@@ -127,22 +130,19 @@ def _shape_like(raster: OwnedRasterArray, t):
 def _shared_layout(*tensors) -> tuple[int, int]:
     """(band stride, row pitch) in elements shared by the given (B, H, W)
     output tensors (None entries skipped); rows must be contiguous."""
-    lay = {(t.stride(0), t.stride(1)) for t in tensors if t is not None}
-    if any(t.stride(2) != 1 for t in tensors if t is not None) or len(lay) > 1:
-        raise ValueError("output tensors must share one (band, row) layout with contiguous rows")
-    return lay.pop() if lay else (0, 0)
+    lay = None
+    for t in tensors:
+        if t is None:
+            continue
+        bs, p, e = t.stride()
+        if e != 1 or (lay is not None and lay != (bs, p)):
+            raise ValueError("output tensors must share one (band, row) layout with contiguous rows")
+        lay = (bs, p)
+    return lay or (0, 0)
 
 
 def _record(result: OwnedRasterArray, detail: str, elapsed: float = 0.0) -> OwnedRasterArray:
-    result.diagnostics.append(
-        RasterDiagnosticEvent(
-            kind=RasterDiagnosticKind.RUNTIME,
-            detail=detail,
-            residency=Residency.DEVICE,
-            visible_to_user=True,
-            elapsed_seconds=elapsed,
-        )
-    )
+    result.diagnostics.append(diagnostic_event(RasterDiagnosticKind.RUNTIME, detail, Residency.DEVICE, True, elapsed))
     return result
 
 
@@ -157,9 +157,7 @@ NODATA_CENTER = "center"  # reference GPU kernel rule (kernels/focal.py:245-250)
 def _terrain_out_dtype(dt: np.dtype) -> np.dtype:
     """float input keeps its dtype, anything else gives float64 (algebra.py:2419-2427)."""
     dt = np.dtype(dt)
-    if np.issubdtype(dt, np.floating) and dt != np.float64:
-        return dt
-    return np.dtype(np.float64)
+    return dt if dt.kind == "f" and dt != _F64 else _F64
 
 
 def horn_fused(
@@ -191,18 +189,19 @@ def horn_fused(
     else:
         flags |= _lib.VSR_HORN_SA_NAN_UNMASKED
     out_np = _terrain_out_dtype(dem.dtype)
-    compute_np = np.dtype(np.float64) if out_np == np.float64 else np.dtype(np.float32)
+    f64 = out_np == np.float64
+    t_dt = torch.float64 if f64 else torch.float32
     o_s, o_a, o_h = out if out is not None else (None, None, None)
     dev = src.device
-    s_t = (o_s if o_s is not None else torch.empty((B, H, W), dtype=torch_dtype(compute_np), device=dev)) if slope else None
-    a_t = (o_a if o_a is not None else torch.empty((B, H, W), dtype=torch_dtype(compute_np), device=dev)) if aspect else None
+    s_t = (o_s if o_s is not None else torch.empty((B, H, W), dtype=t_dt, device=dev)) if slope else None
+    a_t = (o_a if o_a is not None else torch.empty((B, H, W), dtype=t_dt, device=dev)) if aspect else None
     h_t = (o_h if o_h is not None else torch.empty((B, H, W), dtype=torch.uint8, device=dev)) if hillshade else None
     cx, cy = cellsize(dem.affine)
     zen = math.radians(90.0 - float(altitude))
     az = math.radians(float(azimuth))
     lib = _lib.load()
     code = _lib.dtype_code(dt)
-    ocode = _lib.VSR_F64 if compute_np == np.float64 else _lib.VSR_F32
+    ocode = _lib.VSR_F64 if f64 else _lib.VSR_F32
     stream = _stream_handle()
     sa_bs, sa_p = _shared_layout(s_t, a_t)
     h_bs, h_p = _shared_layout(h_t)
@@ -215,7 +214,7 @@ def horn_fused(
         float(z_factor), zen, az, stream,
     )
     _lib.check(st, "vsr_horn_fused_bands")
-    if out_np not in (np.dtype(np.float32), np.dtype(np.float64)):
+    if not f64 and out_np != np.float32:
         s_t = s_t.to(torch_dtype(out_np)) if s_t is not None else None
         a_t = a_t.to(torch_dtype(out_np)) if a_t is not None else None
     return s_t, a_t, h_t

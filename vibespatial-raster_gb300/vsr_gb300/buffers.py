@@ -39,6 +39,14 @@ class RasterDiagnosticEvent:
     bytes_transferred: int = 0
 
 
+def diagnostic_event(kind, detail, residency, visible_to_user=False, elapsed_seconds=0.0) -> RasterDiagnosticEvent:
+    """A RasterDiagnosticEvent without the per-field setattr of a frozen dataclass's __init__ (two per call)."""
+    ev = object.__new__(RasterDiagnosticEvent)
+    ev.__dict__.update(kind=kind, detail=detail, residency=residency, visible_to_user=visible_to_user,
+                       elapsed_seconds=elapsed_seconds, bytes_transferred=0)
+    return ev
+
+
 @dataclass(frozen=True)
 class RasterDeviceState:
     """Device mirror: pixel data and a lazily built boolean nodata mask."""
@@ -47,7 +55,9 @@ class RasterDeviceState:
     nodata_mask: object | None = None
 
 
-_TORCH_TO_NP = None
+_TORCH_OF: dict = {}  # np.dtype -> torch.dtype, built on first use
+_NP_OF: dict = {}     # torch.dtype -> np.dtype
+_NAME_OF: dict = {}   # np.dtype -> str (numpy forms it in Python on each call)
 
 
 def _torch():
@@ -56,39 +66,25 @@ def _torch():
     return torch
 
 
-def torch_dtype(np_dtype):
+def _dtype_tables() -> None:
     torch = _torch()
-    return {
-        np.dtype(np.uint8): torch.uint8,
-        np.dtype(np.int8): torch.int8,
-        np.dtype(np.int16): torch.int16,
-        np.dtype(np.uint16): torch.uint16,
-        np.dtype(np.int32): torch.int32,
-        np.dtype(np.uint32): torch.uint32,
-        np.dtype(np.int64): torch.int64,
-        np.dtype(np.float16): torch.float16,
-        np.dtype(np.float32): torch.float32,
-        np.dtype(np.float64): torch.float64,
-        np.dtype(np.bool_): torch.bool,
-    }[np.dtype(np_dtype)]
+    names = ("uint8", "int8", "int16", "uint16", "int32", "uint32", "int64", "float16", "float32", "float64", "bool")
+    table = {np.dtype(n): getattr(torch, n) for n in names}
+    _NP_OF.update({t: n for n, t in table.items()})
+    _NAME_OF.update({n: str(n) for n in table})
+    _TORCH_OF.update(table)  # in one step: another thread sees none or all
+
+
+def torch_dtype(np_dtype):
+    if not _TORCH_OF:
+        _dtype_tables()
+    return _TORCH_OF[np.dtype(np_dtype)]
 
 
 def numpy_dtype(t_dtype) -> np.dtype:
-    torch = _torch()
-    table = {
-        torch.uint8: np.uint8,
-        torch.int8: np.int8,
-        torch.int16: np.int16,
-        torch.uint16: np.uint16,
-        torch.int32: np.int32,
-        torch.uint32: np.uint32,
-        torch.int64: np.int64,
-        torch.float16: np.float16,
-        torch.float32: np.float32,
-        torch.float64: np.float64,
-        torch.bool: np.bool_,
-    }
-    return np.dtype(table[t_dtype])
+    if not _NP_OF:
+        _dtype_tables()
+    return _NP_OF[t_dtype]
 
 
 def _host_to_device(host: np.ndarray):
@@ -378,14 +374,31 @@ def as_device_tensor(device_data):
     return t
 
 
+_HOLD = bytearray(16)  # one element of any dtype
+
+
+def _host_placeholder(shape: tuple, dtype: np.dtype) -> np.ndarray:
+    """Host array of ``shape`` for a raster whose pixels are on the device only.
+
+    Every element is the same 16 bytes (stride 0): shape, dtype and nbytes read
+    as those of the pixels, which ``to_numpy`` fetches.  Reserving host memory
+    of the raster's size instead cost 67 us per result (map and unmap; 4096^2
+    and larger), more than most of the kernels take.
+    """
+    if 0 in shape:
+        return np.empty(shape, dtype)
+    return np.ndarray(shape, dtype, _HOLD, 0, (0,) * len(shape))
+
+
 def from_device(device_data, *, nodata=None, affine=(1.0, 0.0, 0.0, 0.0, -1.0, 0.0), crs=None) -> OwnedRasterArray:
     """Device-resident raster wrapping a device array without a copy (buffers.py:763-814)."""
     t = as_device_tensor(device_data)
     if t.ndim not in (2, 3):
         raise ValueError(f"raster data must be 2D or 3D, got {t.ndim}D")
     np_dt = numpy_dtype(t.dtype)
+    shape = tuple(t.shape)
     return OwnedRasterArray(
-        data=np.empty(tuple(t.shape), dtype=np_dt),
+        data=_host_placeholder(shape, np_dt),
         nodata=nodata,
         dtype=np_dt,
         affine=tuple(affine),
@@ -394,10 +407,7 @@ def from_device(device_data, *, nodata=None, affine=(1.0, 0.0, 0.0, 0.0, -1.0, 0
         device_state=RasterDeviceState(data=t),
         _host_materialized=False,
         diagnostics=[
-            RasterDiagnosticEvent(
-                kind=RasterDiagnosticKind.CREATED,
-                detail=f"from_device shape={tuple(t.shape)} dtype={np_dt}",
-                residency=Residency.DEVICE,
-            )
+            diagnostic_event(RasterDiagnosticKind.CREATED, f"from_device shape={shape} dtype={_NAME_OF[np_dt]}",
+                             Residency.DEVICE)
         ],
     )
