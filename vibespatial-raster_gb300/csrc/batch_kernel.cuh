@@ -28,23 +28,6 @@ namespace bk {
 
 using namespace horn;
 
-__device__ __forceinline__ bool is_nd_rt(float v, int kind, float ndv) {
-  return kind == VSR_NODATA_VALUE ? (v == ndv) : (kind == VSR_NODATA_NAN ? (v != v) : false);
-}
-
-// Horn rows of one batch item for the tile's nodata kind (warp-uniform).
-template <int RB, bool EDGE, bool VEC>
-__device__ __forceinline__ void batch_horn_rows(const float* S, int lane, int r0, int64_t y0, int64_t xs,
-                                                const HornParams& P, const MaskRule& rule, float nd_in, float* srow,
-                                                float* arow, int64_t sp) {
-  if (P.nd_kind == VSR_NODATA_VALUE)
-    horn_rows<RB, 3, VSR_NODATA_VALUE, EDGE, VEC>(S, lane, r0, y0, xs, P, rule, nd_in, srow, arow, nullptr, sp, sp);
-  else if (P.nd_kind == VSR_NODATA_NAN)
-    horn_rows<RB, 3, VSR_NODATA_NAN, EDGE, VEC>(S, lane, r0, y0, xs, P, rule, nd_in, srow, arow, nullptr, sp, sp);
-  else
-    horn_rows<RB, 3, VSR_NODATA_NONE, EDGE, VEC>(S, lane, r0, y0, xs, P, rule, nd_in, srow, arow, nullptr, sp, sp);
-}
-
 struct BatchTileDev {
   const float* src;
   int64_t H, W, pitch;
@@ -83,29 +66,28 @@ struct BatchSmem {
 };
 
 
-template <int NDK>
-__device__ __forceinline__ bool is_nd_k(float v, float ndv) {
-  if constexpr (NDK == VSR_NODATA_VALUE) return v == ndv;
-  else if constexpr (NDK == VSR_NODATA_NAN) return v != v;
-  else return false;
-}
-
 // The KG x KG Gaussian of one staged item, by each warp for its own RB
 // output rows and its lanes' 4 columns: a horizontal pass per staged row
-// forms (v * valid, valid) pairs with packed FMAs (NaN * 0 stays NaN, as in
-// the reference), a rolling window of the last KG such row sums in
-// registers gives the vertical pass.  No shared memory beyond the staged
-// block and no barrier: the RB + KG - 1 horizontal passes per RB rows cost
-// less than the occupancy a row-sum buffer would take.
-template <int TH, int THREADS, int KG, int NDK, bool VEC>
+// forms (v * valid, valid) sums with packed FMAs (NaN * 0 stays NaN, as in
+// the reference) and adds its terms to the KG - 1 output rows in flight, whose
+// sums move one place per row (acc[j] = g h + acc[j + 1]: an FMA's result may
+// go to another register, so the shift is free).  No shared memory beyond the
+// staged block and no barrier: the RB + KG - 1 horizontal passes per RB rows
+// cost less than the occupancy a row-sum buffer would take.
+//
+// One copy of the row code, not unrolled, for every nodata kind and store
+// width: with all rows unrolled and a copy per variant the kernel outgrew the
+// instruction cache (2.4 of 7.5 cycles per instruction waited for it).
+template <int TH, int THREADS, int KG>
 __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const float (&gw)[KG], int lane, int warp,
-                                            int64_t x0, int64_t y0, int64_t H, int64_t W, float nd_in,
-                                            float nd_out, const BatchTileDev& T) {
+                                            int64_t x0, int64_t y0, int64_t H, int64_t W, float nd_in, int nd_kind,
+                                            float nd_out, float* __restrict__ smooth, int64_t out_pitch, bool vec) {
   using L = BatchSmem<TH, THREADS, KG>;
   constexpr int WARPS = THREADS / 32;
   constexpr int RB = TH / WARPS;
   constexpr int HY = L::HY;
   constexpr int R = KG / 2;
+  constexpr int NA = KG > 1 ? KG - 1 : 1;
   const int c0 = 4 * lane;
   const int q0 = warp * RB;  // first output row of this warp
   // window columns of this lane inside the tile (bit j: column x0 + c0 - R + j)
@@ -122,46 +104,58 @@ __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const f
   const int nrows = static_cast<int>(H - y0 < TH ? H - y0 : int64_t(TH));  // output rows inside the tile
   const int64_t xs = x0 + c0;
   const int ncols = static_cast<int>(W - xs < 4 ? (W - xs > 0 ? W - xs : 0) : 4);
-  float2 win[KG][4];
+  const bool nd_nan = nd_kind == VSR_NODATA_NAN;
+  const float ndq = nd_kind == VSR_NODATA_VALUE ? nd_in : __int_as_float(0x7fffffff);  // NaN: equal to nothing
+  const bool wide = vec && ncols == 4;
+  float* out = smooth + (y0 + q0) * out_pitch + xs;
+  const float* sp = S + (q0 + HY - R) * kSW + c0;  // a lane's window: elements 4 - R .. 7 + R of 12
+  float2 acc[NA][4];
 #pragma unroll
-  for (int i = 0; i < RB + KG - 1; ++i) {
+  for (int j = 0; j < NA; ++j)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[j][u] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+  for (int i = 0; i < RB + KG - 1; ++i, sp += kSW) {
     const int r = q0 + i + HY - R;  // staged row of this horizontal pass
     const uint32_t bits = (r >= first_in && r < rows_in) ? colbits : 0u;
-    const float* sp = S + r * kSW + c0 + 4 - R;
+    const float4 a0 = *reinterpret_cast<const float4*>(sp), a1 = *reinterpret_cast<const float4*>(sp + 4),
+                 a2 = *reinterpret_cast<const float4*>(sp + 8);
+    const float v[12] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
     float2 zv[4 + KG - 1];
 #pragma unroll
     for (int j = 0; j < 4 + KG - 1; ++j) {
-      const float v = sp[j];
-      const bool ok = ((bits >> j) & 1u) && !is_nd_k<NDK>(v, nd_in);
+      const float x = v[4 - R + j];
+      const bool ok = (((bits >> j) & 1u) != 0u) & (x != ndq) & !(nd_nan & (x != x));
       const float o = ok ? 1.0f : 0.0f;
-      zv[j] = make_float2(v * o, o);
+      zv[j] = make_float2(x * o, o);
     }
+    float2 done[4];
 #pragma unroll
-    for (int t = 0; t < KG - 1; ++t)
+    for (int u = 0; u < 4; ++u) {
+      float2 h = make_float2(0.0f, 0.0f);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) win[t][u] = win[t + 1][u];
+      for (int t = 0; t < KG; ++t) h = fma2(f2(gw[t]), zv[u + t], h);
+      if (KG > 1) {
+        done[u] = fma2(f2(gw[KG - 1]), h, acc[0][u]);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) win[KG - 1][u] = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int t = 0; t < KG; ++t) {
-      const float2 w2 = make_float2(gw[t], gw[t]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) win[KG - 1][u] = fma2(w2, zv[u + t], win[KG - 1][u]);
+        for (int j = 0; j + 1 < KG - 1; ++j) acc[j][u] = fma2(f2(gw[KG - 2 - j]), h, acc[j + 1][u]);
+        acc[NA - 1][u] = mul2(f2(gw[0]), h);
+      } else {
+        done[u] = fma2(f2(gw[0]), h, make_float2(0.0f, 0.0f));
+      }
     }
     if (i >= KG - 1) {
-      const int q = q0 + i - (KG - 1);  // output row
-      if (q < nrows && ncols > 0) {
+      if (q0 + i - (KG - 1) < nrows && ncols > 0) {
+        const float4 c4 = *reinterpret_cast<const float4*>(sp - (KG - 1 - R) * kSW + 4);  // the centres
+        const float cv[4] = {c4.x, c4.y, c4.z, c4.w};
         float o4[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          float2 acc = make_float2(0.0f, 0.0f);
-#pragma unroll
-          for (int t = 0; t < KG; ++t) acc = fma2(make_float2(gw[t], gw[t]), win[t][u], acc);
-          const bool centre_ok = !is_nd_k<NDK>(S[(q + HY) * kSW + c0 + 4 + u], nd_in);
-          o4[u] = (centre_ok && acc.y > 0.0f) ? __fdividef(acc.x, acc.y) : nd_out;
+          const bool ok = (cv[u] != ndq) & !(nd_nan & (cv[u] != cv[u])) & (done[u].y > 0.0f);
+          const float q = __fdividef(done[u].x, done[u].y);
+          o4[u] = ok ? q : nd_out;
         }
-        float* out = T.smooth + (y0 + q) * T.out_pitch + xs;
-        if (VEC && ncols == 4) {
+        if (wide) {
           __stcs(reinterpret_cast<float4*>(out), make_float4(o4[0], o4[1], o4[2], o4[3]));
         } else {
 #pragma unroll
@@ -169,6 +163,7 @@ __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const f
             if (u < ncols) out[u] = o4[u];
         }
       }
+      out += out_pitch;
     }
   }
 }
@@ -328,27 +323,22 @@ __global__ void __launch_bounds__(THREADS) batch_terrain_kernel(BatchHeader* __r
       const RowPtrs g = global_rows(T.slope, T.aspect, nullptr, P, y0 + warp * RB, xs);
       // both outputs are requested together in the batch plan
       if (T.vec) {
-        if (edge) batch_horn_rows<RB, true, true>(Sh, lane, warp * RB, y0, xs, P, rule, nd_in, g.s, g.a, P.out_pitch);
-        else batch_horn_rows<RB, false, true>(Sh, lane, warp * RB, y0, xs, P, rule, nd_in, g.s, g.a, P.out_pitch);
+        if (edge)
+          horn_rows<RB, 3, kNdRuntime, true, true>(Sh, lane, warp * RB, y0, xs, P, rule, nd_in, g.s, g.a, nullptr,
+                                                   P.out_pitch, P.out_pitch);
+        else
+          horn_rows<RB, 3, kNdRuntime, false, true>(Sh, lane, warp * RB, y0, xs, P, rule, nd_in, g.s, g.a, nullptr,
+                                                    P.out_pitch, P.out_pitch);
       } else {
-        batch_horn_rows<RB, true, false>(Sh, lane, warp * RB, y0, xs, P, rule, nd_in, g.s, g.a, P.out_pitch);
+        horn_rows<RB, 3, kNdRuntime, true, false>(Sh, lane, warp * RB, y0, xs, P, rule, nd_in, g.s, g.a, nullptr,
+                                                  P.out_pitch, P.out_pitch);
       }
     }
 
     // Gaussian KG x KG (normalised, nodata-aware, out-of-bounds taps skipped).
-    if (T.smooth) {
-      const bool vec = T.vec_smooth != 0;
-      if (P.nd_kind == VSR_NODATA_VALUE) {
-        if (vec) batch_gauss<TH, THREADS, KG, VSR_NODATA_VALUE, true>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T);
-        else batch_gauss<TH, THREADS, KG, VSR_NODATA_VALUE, false>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T);
-      } else if (P.nd_kind == VSR_NODATA_NAN) {
-        if (vec) batch_gauss<TH, THREADS, KG, VSR_NODATA_NAN, true>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T);
-        else batch_gauss<TH, THREADS, KG, VSR_NODATA_NAN, false>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T);
-      } else {
-        if (vec) batch_gauss<TH, THREADS, KG, VSR_NODATA_NONE, true>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T);
-        else batch_gauss<TH, THREADS, KG, VSR_NODATA_NONE, false>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T);
-      }
-    }
+    if (T.smooth)
+      batch_gauss<TH, THREADS, KG>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_kind, P.nd_out_f, T.smooth, P.out_pitch,
+                                   T.vec_smooth != 0);
     __syncthreads();  // every read of buffer b and of its item slots is done before they are reassigned
   }
   cp_async_wait<0>();  // no copy may land after the CTA leaves
@@ -369,9 +359,9 @@ int launch_batch_t(BatchHeader* hdr, const BatchTileDev* tiles, cudaStream_t st)
   if (!err) return VSR_ERR_CUDA;
   const size_t smem = static_cast<size_t>(L::kFloats) * 4;
   auto kern = batch_terrain_kernel<TH, THREADS, KG>;
-  VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  static KernelResidency residency;
   int per_sm = 0;
-  VSR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem));
+  VSR_CUDA_TRY(residency.get(kern, THREADS, smem, &per_sm));
   if (per_sm < 1) return fail(VSR_ERR_CUDA, "batch kernel cannot be resident");
   kern<<<static_cast<unsigned>(sm_count() * per_sm), THREADS, smem, st>>>(hdr, tiles, err);
   VSR_CUDA_TRY(cudaGetLastError());

@@ -1110,61 +1110,48 @@ struct Vec4Of<uint8_t> {
   using type = uint32_t;
 };
 
-template <int R, typename T, bool VOUT, bool F64>
-__global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
-  static_assert(R >= 1 && R <= 4, "the neighbour exchange covers radii up to 4");
+template <int R, typename T, bool VOUT, bool F64, bool EDGE>
+__device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __restrict__ tab, int64_t xw) {
   using Pk = SlidePack<R>;
   using V4 = typename Vec4Of<T>::type;
   constexpr int P = 2 * R + 1;
   constexpr bool kByte = sizeof(T) == 1;
   constexpr int OFF = std::is_signed<T>::value ? 32768 : 0;
   constexpr uint32_t kOne = 1u << Pk::kShift, kLow = kOne - 1u;
-  static_assert(Pk::kShift >= 16 && Pk::kShift <= 23, "the count bit sits in byte 2; value sums stay below 2^23");
   // int16 values + 32768 = their bits with bit 15 flipped
   constexpr uint32_t kFlip = OFF ? 0x80008000u : 0u;
-  __shared__ float2 tab[Pk::kTaps + 1];  // (RN(1/n), -n)
-  for (int i = threadIdx.x; i <= Pk::kTaps; i += blockDim.x)
-    tab[i] = make_float2(i ? __frcp_rn(static_cast<float>(i)) : 0.0f, -static_cast<float>(i));
-  __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int64_t xw = (static_cast<int64_t>(blockIdx.x) * kBwWarps + (threadIdx.x >> 5)) * kBwCols;
-  if (xw >= a.W) return;  // the whole warp: no block-wide barrier follows
   const int64_t xs = xw - 4 + 4 * lane;  // this lane's first column (a multiple of 4)
   const int64_t ys = static_cast<int64_t>(blockIdx.y) * kBwStrip;
   const T* src = static_cast<const T*>(band_src(a.src, a.dtype, a.band_stride));
   void* dst = band_dst(a.dst, a.out_dtype, a.out_band_stride);
   const int nout = static_cast<int>(a.H - ys < kBwStrip ? a.H - ys : kBwStrip);
   const int nin = nout + 2 * R;  // input rows ys - R .. ys + nout + R - 1
-  const bool has_nd = a.nd.kind == VSR_NODATA_VALUE;
-  // the nodata value's bit pattern in every element slot of a word
-  const uint32_t ndp = static_cast<uint32_t>(a.nd.iv) & (kByte ? 0xFFu : 0xFFFFu);
-  const uint32_t nd_word = kByte ? ndp * 0x01010101u : ndp * 0x00010001u;
-  // elements of the group inside [0, W), as byte (8-bit) or half-word masks
-  // of the two words; one vector load per group inside the raster, element
-  // loads for the group that straddles column W
-  uint32_t cmx = 0u, cmy = 0u;
+  // input rows [r0, r1) lie in the raster
+  const int r0 = ys < R ? static_cast<int>(R - ys) : 0;
+  const int r1 = a.H - (ys - R) < nin ? static_cast<int>(a.H - (ys - R)) : nin;
+  // the nodata value as a packed word; no word equals 0xFFFFFFFF
+  const uint32_t ndw = a.nd.kind == VSR_NODATA_VALUE
+                           ? kOne | ((static_cast<uint32_t>(a.nd.iv) ^ (kFlip & 0xFFFFu)) & (kByte ? 0xFFu : 0xFFFFu))
+                           : 0xFFFFFFFFu;
+  bool in[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const uint32_t in = (xs + e >= 0 && xs + e < a.W) ? 1u : 0u;
-    if (kByte) cmx |= (in * 0xFFu) << (8 * e);
-    else if (e < 2) cmx |= (in * 0xFFFFu) << (16 * e);
-    else cmy |= (in * 0xFFFFu) << (16 * (e - 2));
-  }
-  const bool ld = xs >= 0 && xs < a.W, whole = xs >= 0 && xs + 4 <= a.W;
-  const bool out_lane = lane >= 1 && lane <= kBwLanes;
+  for (int e = 0; e < 4; ++e) in[e] = xs + e >= 0 && xs + e < a.W;
+  const bool out_lane = lane >= 1 && lane <= kBwLanes && in[0];
+  const bool vec = VOUT && in[3];
 
   // input row i is raster row ys - R + i; its pointer steps by the pitch
   const T* rp = src + (ys - R) * a.pitch + xs;
   auto load = [&](int i, const T* p) -> V4 {
-    const uint64_t gy = static_cast<uint64_t>(ys - R + i);
     V4 v{};
-    if (ld && i < nin && gy < static_cast<uint64_t>(a.H)) {
-      if (whole) {
-        v = __ldg(reinterpret_cast<const V4*>(p));
+    if (i >= r0 && i < r1) {
+      if (!EDGE || in[3]) {
+        if (!EDGE || in[0]) v = __ldg(reinterpret_cast<const V4*>(p));
       } else {
         uint32_t e[4] = {0u, 0u, 0u, 0u};
-        for (int q = 0; q < 4 && xs + q < a.W; ++q)
-          e[q] = static_cast<uint32_t>(static_cast<std::make_unsigned_t<T>>(__ldg(p + q)));
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (in[q]) e[q] = static_cast<uint32_t>(static_cast<std::make_unsigned_t<T>>(__ldg(p + q)));
         if constexpr (kByte) v = e[0] | (e[1] << 8) | (e[2] << 16) | (e[3] << 24);
         else v = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
       }
@@ -1176,7 +1163,7 @@ __global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
   for (int u = 0; u < P; ++u) pre[u] = load(u, rp + u * a.pitch);
   const T* lp = rp + P * a.pitch;  // the row P ahead
   uint32_t hs[P][4];  // horizontal sums of the last P rows (ring slot = row % P)
-  uint32_t vm[P];     // their validity, one byte per element (0xFF valid)
+  uint32_t vm[P];     // their validity: byte e holds element e's count bit
 #pragma unroll
   for (int u = 0; u < P; ++u) {
     vm[u] = 0u;
@@ -1185,7 +1172,8 @@ __global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
   }
   uint32_t V[4] = {0u, 0u, 0u, 0u};
   const float ndf = static_cast<float>(a.nd_out);
-  int64_t orow = ys * a.out_pitch + xs;  // output row i - 2R
+  char* op = static_cast<char*>(dst) + (ys * a.out_pitch + xs) * (F64 ? 8 : 4);
+  const int64_t ostep = a.out_pitch * (F64 ? 8 : 4);
   // correctly rounded sum / count for two columns: q0 = fs / n by the
   // reciprocal, one FMA residual correction (exact integers in float32)
   auto quot2 = [&](uint32_t va, uint32_t vb) -> float2 {
@@ -1205,37 +1193,37 @@ __global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
       const V4 raw = pre[u];
       pre[u] = load(i + P, lp);
       lp += a.pitch;
-      const uint32_t rowm = static_cast<uint64_t>(ys - R + i) < static_cast<uint64_t>(a.H) ? 0xFFFFFFFFu : 0u;
       // packed words: the element (plus the offset) in bits 0-15, the count
-      // bit above, or 0 where invalid -- byte permutes of the raw words
+      // bit above, or 0 where invalid
       uint32_t w[12];  // left neighbour's 4 words, this lane's, the right neighbour's
-      uint32_t m;      // validity, one byte per element
-      if constexpr (kByte) {
-        const uint32_t x = raw;
-        uint32_t k = cmx & rowm;
-        if (has_nd) k &= ~__vcmpeq4(x, nd_word);
-        m = k;
-        w[4] = __byte_perm(x, kOne, 0x7640) & __byte_perm(k, 0u, 0x0000);
-        w[5] = __byte_perm(x, kOne, 0x7641) & __byte_perm(k, 0u, 0x1111);
-        w[6] = __byte_perm(x, kOne, 0x7642) & __byte_perm(k, 0u, 0x2222);
-        w[7] = __byte_perm(x, kOne, 0x7643) & __byte_perm(k, 0u, 0x3333);
-      } else {
-        const uint32_t x = raw.x, y = raw.y;  // (v0 | v1 << 16), (v2 | v3 << 16)
-        uint32_t kx = cmx & rowm, ky = cmy & rowm;
-        if (has_nd) {
-          kx &= ~__vcmpeq2(x, nd_word);
-          ky &= ~__vcmpeq2(y, nd_word);
+      if (i >= r0 && i < r1) {
+        if constexpr (kByte) {
+          w[4] = __byte_perm(raw, kOne, 0x7640);
+          w[5] = __byte_perm(raw, kOne, 0x7641);
+          w[6] = __byte_perm(raw, kOne, 0x7642);
+          w[7] = __byte_perm(raw, kOne, 0x7643);
+        } else {
+          const uint32_t x = raw.x ^ kFlip, y = raw.y ^ kFlip;  // (v0 | v1 << 16), (v2 | v3 << 16)
+          w[4] = __byte_perm(x, kOne, 0x7610);
+          w[5] = __byte_perm(x, kOne, 0x7632);
+          w[6] = __byte_perm(y, kOne, 0x7610);
+          w[7] = __byte_perm(y, kOne, 0x7632);
         }
-        m = __byte_perm(kx, ky, 0x6420);
-        w[4] = __byte_perm(x ^ kFlip, kOne, 0x7610) & __byte_perm(kx, 0u, 0x1010);
-        w[5] = __byte_perm(x ^ kFlip, kOne, 0x7632) & __byte_perm(kx, 0u, 0x3232);
-        w[6] = __byte_perm(y ^ kFlip, kOne, 0x7610) & __byte_perm(ky, 0u, 0x1010);
-        w[7] = __byte_perm(y ^ kFlip, kOne, 0x7632) & __byte_perm(ky, 0u, 0x3232);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          w[4 + e] = w[4 + e] == ndw ? 0u : w[4 + e];
+          if (EDGE) w[4 + e] = in[e] ? w[4 + e] : 0u;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[4 + e] = 0u;
       }
+      // the count bits (byte 2 of each word)
+      vm[u] = __byte_perm(__byte_perm(w[4], w[5], 0x0062), __byte_perm(w[6], w[7], 0x0062), 0x5410);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        w[e] = __shfl_up_sync(0xffffffffu, w[4 + e], 1);
-        w[8 + e] = __shfl_down_sync(0xffffffffu, w[4 + e], 1);
+        if (e >= 4 - R) w[e] = __shfl_up_sync(0xffffffffu, w[4 + e], 1);
+        if (e < R) w[8 + e] = __shfl_down_sync(0xffffffffu, w[4 + e], 1);
       }
       uint32_t h = 0u;
 #pragma unroll
@@ -1246,37 +1234,51 @@ __global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
         V[c] += h - hs[u][c];
         hs[u][c] = h;
       }
-      vm[u] = m;
       if (i >= 2 * R) {
         if (out_lane) {
           const uint32_t cm = vm[(u + P - R) % P];  // the centre row i - R
+          constexpr uint32_t kBit = kOne >> 16;     // the count bit within its byte
           if constexpr (F64) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
               const int cnt = static_cast<int>(V[c] >> Pk::kShift);
               const int sum = static_cast<int>(V[c] & kLow) - OFF * cnt;
-              if (xs + c < a.W)
-                static_cast<double*>(dst)[orow + c] =
-                    ((cm >> (8 * c)) & 1u) ? static_cast<double>(sum) / static_cast<double>(cnt) : a.nd_out;
+              if (in[c])
+                reinterpret_cast<double*>(op)[c] =
+                    (cm & (kBit << (8 * c))) ? static_cast<double>(sum) / static_cast<double>(cnt) : a.nd_out;
             }
           } else {
             const float2 q01 = quot2(V[0], V[1]), q23 = quot2(V[2], V[3]);
-            const float q[4] = {(cm & 1u) ? q01.x : ndf, ((cm >> 8) & 1u) ? q01.y : ndf,
-                                ((cm >> 16) & 1u) ? q23.x : ndf, ((cm >> 24) & 1u) ? q23.y : ndf};
-            float* op = static_cast<float*>(dst) + orow;
-            if (VOUT && xs + 3 < a.W) {
+            const float q[4] = {(cm & kBit) ? q01.x : ndf, (cm & (kBit << 8)) ? q01.y : ndf,
+                                (cm & (kBit << 16)) ? q23.x : ndf, (cm & (kBit << 24)) ? q23.y : ndf};
+            if (vec) {
               *reinterpret_cast<float4*>(op) = make_float4(q[0], q[1], q[2], q[3]);
             } else {
 #pragma unroll
               for (int c = 0; c < 4; ++c)
-                if (xs + c < a.W) op[c] = q[c];
+                if (in[c]) reinterpret_cast<float*>(op)[c] = q[c];
             }
           }
         }
-        orow += a.out_pitch;
+        op += ostep;
       }
     }
   }
+}
+
+template <int R, typename T, bool VOUT, bool F64>
+__global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
+  static_assert(R >= 1 && R <= 4, "the neighbour exchange covers radii up to 4");
+  using Pk = SlidePack<R>;
+  static_assert(Pk::kShift >= 16 && Pk::kShift <= 23, "the count bit sits in byte 2; value sums stay below 2^23");
+  __shared__ float2 tab[Pk::kTaps + 1];  // (RN(1/n), -n)
+  for (int i = threadIdx.x; i <= Pk::kTaps; i += blockDim.x)
+    tab[i] = make_float2(i ? __frcp_rn(static_cast<float>(i)) : 0.0f, -static_cast<float>(i));
+  __syncthreads();
+  const int64_t xw = (static_cast<int64_t>(blockIdx.x) * kBwWarps + (threadIdx.x >> 5)) * kBwCols;
+  if (xw >= a.W) return;  // the whole warp: no block-wide barrier follows
+  if (xw >= 4 && xw + 124 <= a.W) box_strip<R, T, VOUT, F64, false>(a, tab, xw);
+  else box_strip<R, T, VOUT, F64, true>(a, tab, xw);
 }
 
 template <int R, typename T>

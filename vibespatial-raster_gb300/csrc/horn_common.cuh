@@ -283,11 +283,19 @@ __device__ __forceinline__ void stage_row(const float* row, int lane, Row& r) {
   r.hi = fmaxf(max3f(r.v[0], r.v[1], r.v[2]), max3f(r.v[3], r.v[4], r.v[5]));
 }
 
+// Nodata kind known at run time only (P.nd_kind): one copy of the row code for
+// tiles of every kind.
+constexpr int kNdRuntime = 3;
+
 // Could the row hold nodata?  A value nodata can only be present if it lies
 // within the row's range; a NaN anywhere makes a difference NaN (inf - inf
 // also does: a harmless false alarm).
 template <int NDK>
-__device__ __forceinline__ bool row_may_hold_nodata(const Row& r, float ndv) {
+__device__ __forceinline__ bool row_may_hold_nodata(const Row& r, float ndv, int kind) {
+  if (NDK == kNdRuntime) {
+    const float s = (r.hd[0] + r.hd[1]) + (r.hd[2] + r.hd[3]);
+    return ((kind == VSR_NODATA_VALUE) & (ndv >= r.lo) & (ndv <= r.hi)) | ((kind == VSR_NODATA_NAN) & (s != s));
+  }
   if (NDK == VSR_NODATA_VALUE) return ndv >= r.lo && ndv <= r.hi;
   if (NDK == VSR_NODATA_NAN) {
     const float s = (r.hd[0] + r.hd[1]) + (r.hd[2] + r.hd[3]);
@@ -297,17 +305,18 @@ __device__ __forceinline__ bool row_may_hold_nodata(const Row& r, float ndv) {
 }
 
 template <int NDK>
-__device__ __forceinline__ bool is_nd(float v, float ndv) {
+__device__ __forceinline__ bool is_nd(float v, float ndv, int kind) {
+  if (NDK == kNdRuntime) return ((kind == VSR_NODATA_VALUE) & (v == ndv)) | ((kind == VSR_NODATA_NAN) & (v != v));
   return NDK == VSR_NODATA_VALUE ? (v == ndv) : (NDK == VSR_NODATA_NAN ? (v != v) : false);
 }
 
 // Nodata bits of a row's 6 values; with ``skip`` its range is narrowed to the
 // valid values (outputs whose windows hold nodata are masked anyway).
 template <int NDK>
-__device__ __forceinline__ uint32_t row_nodata(Row& r, float ndv, bool skip) {
+__device__ __forceinline__ uint32_t row_nodata(Row& r, float ndv, int kind, bool skip) {
   uint32_t m = 0;
 #pragma unroll
-  for (int k = 0; k < 6; ++k) m |= (is_nd<NDK>(r.v[k], ndv) ? 1u : 0u) << k;
+  for (int k = 0; k < 6; ++k) m |= (is_nd<NDK>(r.v[k], ndv, kind) ? 1u : 0u) << k;
   if (skip && m) {
     float l[6], h[6];
 #pragma unroll
@@ -421,22 +430,22 @@ __device__ __forceinline__ void horn_rows(const float* S, int lane, int r0, int6
   Row r0v, r1v;
   stage_row(S + (r0 + 0) * kSW, lane, r0v);
   stage_row(S + (r0 + 1) * kSW, lane, r1v);
-  bool f0 = row_may_hold_nodata<NDK>(r0v, nd_in), f1 = row_may_hold_nodata<NDK>(r1v, nd_in);
+  bool f0 = row_may_hold_nodata<NDK>(r0v, nd_in, P.nd_kind), f1 = row_may_hold_nodata<NDK>(r1v, nd_in, P.nd_kind);
   const int64_t y = y0 + r0;
 #pragma unroll 1
   for (int j = 0; j < RB; j += 2) {
     Row r2v, r3v;
     stage_row(S + (r0 + j + 2) * kSW, lane, r2v);
     stage_row(S + (r0 + j + 3) * kSW, lane, r3v);
-    const bool f2 = row_may_hold_nodata<NDK>(r2v, nd_in), f3 = row_may_hold_nodata<NDK>(r3v, nd_in);
+    const bool f2 = row_may_hold_nodata<NDK>(r2v, nd_in, P.nd_kind), f3 = row_may_hold_nodata<NDK>(r3v, nd_in, P.nd_kind);
     const bool masked = NDK != VSR_NODATA_NONE && __any_sync(0xffffffffu, f0 | f1 | f2 | f3);
     uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
     Row a = r0v, b = r1v, c = r2v, d = r3v;  // ranges narrowed to valid values when masked
     if (masked) {
-      m0 = row_nodata<NDK>(a, nd_in, skip_nd);
-      m1 = row_nodata<NDK>(b, nd_in, skip_nd);
-      m2 = row_nodata<NDK>(c, nd_in, skip_nd);
-      m3 = row_nodata<NDK>(d, nd_in, skip_nd);
+      m0 = row_nodata<NDK>(a, nd_in, P.nd_kind, skip_nd);
+      m1 = row_nodata<NDK>(b, nd_in, P.nd_kind, skip_nd);
+      m2 = row_nodata<NDK>(c, nd_in, P.nd_kind, skip_nd);
+      m3 = row_nodata<NDK>(d, nd_in, P.nd_kind, skip_nd);
     }
     // both output rows of the pair take the exact form if any lane's window may round
     const float lo = fminf(min3f(a.lo, b.lo, c.lo), d.lo), hi = fmaxf(max3f(a.hi, b.hi, c.hi), d.hi);
