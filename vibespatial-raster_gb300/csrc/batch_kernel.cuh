@@ -4,6 +4,8 @@
 // Gaussian width so that they compile in parallel.
 #pragma once
 
+#include <type_traits>
+
 #include "horn_common.cuh"
 
 // One persistent, work-queue-scheduled launch over many DEM tiles of uneven
@@ -75,12 +77,21 @@ struct BatchSmem {
 // staged block and no barrier: the RB + KG - 1 horizontal passes per RB rows
 // cost less than the occupancy a row-sum buffer would take.
 //
-// One copy of the row code, not unrolled, for every nodata kind and store
-// width: with all rows unrolled and a copy per variant the kernel outgrew the
-// instruction cache (2.4 of 7.5 cycles per instruction waited for it).
-template <int TH, int THREADS, int KG>
+// The rows are not unrolled: with all of them unrolled per nodata kind and
+// store width the kernel outgrew the instruction cache (2.4 of 7.5 cycles per
+// instruction waited for it).  The ALU pipe is the busiest (compares, selects
+// and min / max run there at half the rate of FMAs), so a tap inside the tile
+// (not EDGE) takes one compare.
+template <int NDK>
+__device__ __forceinline__ bool tap_valid(float v, float ndv) {
+  if constexpr (NDK == VSR_NODATA_VALUE) return v != ndv;
+  else if constexpr (NDK == VSR_NODATA_NAN) return v == v;
+  else return true;
+}
+
+template <int TH, int THREADS, int KG, int NDK, bool EDGE>
 __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const float (&gw)[KG], int lane, int warp,
-                                            int64_t x0, int64_t y0, int64_t H, int64_t W, float nd_in, int nd_kind,
+                                            int64_t x0, int64_t y0, int64_t H, int64_t W, float nd_in,
                                             float nd_out, float* __restrict__ smooth, int64_t out_pitch, bool vec) {
   using L = BatchSmem<TH, THREADS, KG>;
   constexpr int WARPS = THREADS / 32;
@@ -104,8 +115,6 @@ __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const f
   const int nrows = static_cast<int>(H - y0 < TH ? H - y0 : int64_t(TH));  // output rows inside the tile
   const int64_t xs = x0 + c0;
   const int ncols = static_cast<int>(W - xs < 4 ? (W - xs > 0 ? W - xs : 0) : 4);
-  const bool nd_nan = nd_kind == VSR_NODATA_NAN;
-  const float ndq = nd_kind == VSR_NODATA_VALUE ? nd_in : __int_as_float(0x7fffffff);  // NaN: equal to nothing
   const bool wide = vec && ncols == 4;
   float* out = smooth + (y0 + q0) * out_pitch + xs;
   const float* sp = S + (q0 + HY - R) * kSW + c0;  // a lane's window: elements 4 - R .. 7 + R of 12
@@ -125,7 +134,7 @@ __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const f
 #pragma unroll
     for (int j = 0; j < 4 + KG - 1; ++j) {
       const float x = v[4 - R + j];
-      const bool ok = (((bits >> j) & 1u) != 0u) & (x != ndq) & !(nd_nan & (x != x));
+      const bool ok = (!EDGE | (((bits >> j) & 1u) != 0u)) & tap_valid<NDK>(x, nd_in);
       const float o = ok ? 1.0f : 0.0f;
       zv[j] = make_float2(x * o, o);
     }
@@ -151,7 +160,7 @@ __device__ __forceinline__ void batch_gauss(const float* __restrict__ S, const f
         float o4[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const bool ok = (cv[u] != ndq) & !(nd_nan & (cv[u] != cv[u])) & (done[u].y > 0.0f);
+          const bool ok = tap_valid<NDK>(cv[u], nd_in) & (done[u].y > 0.0f);
           const float q = __fdividef(done[u].x, done[u].y);
           o4[u] = ok ? q : nd_out;
         }
@@ -336,9 +345,21 @@ __global__ void __launch_bounds__(THREADS) batch_terrain_kernel(BatchHeader* __r
     }
 
     // Gaussian KG x KG (normalised, nodata-aware, out-of-bounds taps skipped).
-    if (T.smooth)
-      batch_gauss<TH, THREADS, KG>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_kind, P.nd_out_f, T.smooth, P.out_pitch,
-                                   T.vec_smooth != 0);
+    if (T.smooth) {
+      const bool whole = x0 >= 4 && x0 + kTW + 4 <= W && y0 >= HY && y0 + TH + HY <= H;  // every tap in the tile
+      auto run = [&](auto ndk) {
+        constexpr int NDK = decltype(ndk)::value;
+        if (whole)
+          batch_gauss<TH, THREADS, KG, NDK, false>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T.smooth,
+                                                   P.out_pitch, T.vec_smooth != 0);
+        else
+          batch_gauss<TH, THREADS, KG, NDK, true>(S, gw, lane, warp, x0, y0, H, W, nd_in, P.nd_out_f, T.smooth,
+                                                  P.out_pitch, T.vec_smooth != 0);
+      };
+      if (P.nd_kind == VSR_NODATA_VALUE) run(std::integral_constant<int, VSR_NODATA_VALUE>{});
+      else if (P.nd_kind == VSR_NODATA_NAN) run(std::integral_constant<int, VSR_NODATA_NAN>{});
+      else run(std::integral_constant<int, VSR_NODATA_NONE>{});
+    }
     __syncthreads();  // every read of buffer b and of its item slots is done before they are reassigned
   }
   cp_async_wait<0>();  // no copy may land after the CTA leaves
