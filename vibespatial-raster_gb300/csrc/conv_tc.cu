@@ -240,6 +240,33 @@ __device__ __noinline__ float inf_window(const float* __restrict__ src, int64_t 
   return pos ? __int_as_float(0x7f800000) : __int_as_float(0xff800000);
 }
 
+// The MMAs of one kernel row, KS k-steps (4 for single columns, 5..7 up to
+// kMaxTCK) without a loop.  With the warp kept uniform (elect_one) a further
+// MMA costs 23 ns from 21x21 to 31x31 and 28 ns on to 41x41 (time of a tile
+// over the MMAs added), 35 and 34 ns before.
+template <int KS>
+__device__ __forceinline__ void issue_row(uint32_t tg, uint32_t t_corr, uint32_t td, uint32_t ah, uint32_t al,
+                                          uint32_t av, uint32_t bh, uint32_t bl, uint32_t bf, uint32_t a_ks,
+                                          uint32_t f, uint32_t fc, bool den_mma) {
+  if (den_mma) {
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      mma_bf16(tg, ah + ks * a_ks, bh + ks * 16, ks ? 1u : f);
+      mma_bf16(t_corr, ah + ks * a_ks, bl + ks * 16, ks ? 1u : fc);
+      mma_f16(t_corr, al + ks * a_ks, bf + ks * 16, 1u);
+      mma_bf16(td, av + ks * a_ks, bh + ks * 16, ks ? 1u : f);
+      mma_bf16(td, av + ks * a_ks, bl + ks * 16, 1u);
+    }
+  } else {
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      mma_bf16(tg, ah + ks * a_ks, bh + ks * 16, ks ? 1u : f);
+      mma_bf16(t_corr, ah + ks * a_ks, bl + ks * 16, ks ? 1u : fc);
+      mma_f16(t_corr, al + ks * a_ks, bf + ks * 16, 1u);
+    }
+  }
+}
+
 // ND: the raster's nodata rule (0 none, 1 a value, 2 NaN).
 template <int ND>
 __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, uint32_t* err_word) {
@@ -254,7 +281,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, 
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
   const TcGeom g = make_geom(a.kh, a.kw);
   const TcPlan L = make_plan(g, ND != 0, a.nbuf, a.nst);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // value scale zs = 2^(14 - E) for a largest |value| below 2^E: |v - mu| < 2^15
   int zexp = 0;
   {
@@ -310,38 +337,40 @@ __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, 
 
   if (warp == 0) {
     // ========================================================= MMA issuer
-    if (lane == 0) {
-      const uint32_t lbo_a = static_cast<uint32_t>(g.Rp) * 16;
-      const uint32_t a_ks = (2 * lbo_a) >> 4;  // one k-step = two core matrices along K
-      const uint32_t w_ring = desc_lo(s_base + L.ring, 128), stage_w = L.stage_bytes >> 4, row_w = L.row_bytes >> 4;
-      // first kernel rows of accumulator groups 1 and 2 (kh when absent):
-      // row ky belongs to group floor(ky G / kh)
-      const int gb1 = g.G > 1 ? (a.kh + g.G - 1) / g.G : a.kh;
-      const int gb2 = g.G > 2 ? (2 * a.kh + g.G - 1) / g.G : a.kh;
-      uint32_t u = 0;                          // band-ring uses
-      int j = 0;
-      bool ok = true;
-      for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++j) {
-        const int b = j % a.nbuf, tb = j % L.tbuf, slot = j & 1;
-        ok = wait_or_abort(&a_full[b], (j / a.nbuf) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
-        if (ok && j >= L.tbuf)
-          ok = wait_or_abort(&acc_empty[tb], ((j / L.tbuf) - 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+    const uint32_t lbo_a = static_cast<uint32_t>(g.Rp) * 16;
+    const uint32_t a_ks = (2 * lbo_a) >> 4;  // one k-step = two core matrices along K
+    const uint32_t w_ring = desc_lo(s_base + L.ring, 128), stage_w = L.stage_bytes >> 4, row_w = L.row_bytes >> 4;
+    // first kernel rows of accumulator groups 1 and 2 (kh when absent):
+    // row ky belongs to group floor(ky G / kh)
+    const int gb1 = g.G > 1 ? (a.kh + g.G - 1) / g.G : a.kh;
+    const int gb2 = g.G > 2 ? (2 * a.kh + g.G - 1) / g.G : a.kh;
+    uint32_t u = 0;                          // band-ring uses
+    int j = 0;
+    bool ok = true;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+      const int b = j % a.nbuf, tb = j % L.tbuf, slot = j & 1;
+      ok = wait_or_abort(&a_full[b], (j / a.nbuf) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+      if (ok && j >= L.tbuf)
+        ok = wait_or_abort(&acc_empty[tb], ((j / L.tbuf) - 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const bool den_mma = info_nd[slot] != 0;
+      const uint32_t w_ahi = desc_lo(s_base + L.a_hi + b * L.a_bytes, lbo_a);
+      const uint32_t w_alo = desc_lo(s_base + L.a_lo + b * L.a_bytes, lbo_a);
+      const uint32_t w_avd = desc_lo(s_base + L.a_vd + b * L.a_bytes, lbo_a);
+      const uint32_t t_acc = tmem + tb * L.cols;
+      const uint32_t t_corr = t_acc + g.G * kTN, t_den = t_acc + (g.G + 1) * kTN;
+      // Per ring stage one wait and one release; per kernel row a few
+      // integer ops, then the MMAs (the thread's overhead between rows is
+      // time the tensor pipe may run dry).  The band-full wait needs no
+      // tcgen05 fence: the copy completes on the mbarrier itself.
+      for (int ky0 = 0; ky0 < a.kh; ky0 += kRowsPerStage, ++u) {
+        const uint32_t s = u % L.nst;
+        ok = wait_or_abort(&b_full[s], (u / L.nst) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        tc_fence_after();
-        const bool den_mma = info_nd[slot] != 0;
-        const uint32_t w_ahi = desc_lo(s_base + L.a_hi + b * L.a_bytes, lbo_a);
-        const uint32_t w_alo = desc_lo(s_base + L.a_lo + b * L.a_bytes, lbo_a);
-        const uint32_t w_avd = desc_lo(s_base + L.a_vd + b * L.a_bytes, lbo_a);
-        const uint32_t t_acc = tmem + tb * L.cols;
-        const uint32_t t_corr = t_acc + g.G * kTN, t_den = t_acc + (g.G + 1) * kTN;
-        // Per ring stage one wait and one release; per kernel row a few
-        // integer ops, then the MMAs (the thread's overhead between rows is
-        // time the tensor pipe may run dry).  The band-full wait needs no
-        // tcgen05 fence: the copy completes on the mbarrier itself.
-        for (int ky0 = 0; ky0 < a.kh; ky0 += kRowsPerStage, ++u) {
-          const uint32_t s = u % L.nst;
-          ok = wait_or_abort(&b_full[s], (u / L.nst) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
-          if (!ok) break;
+        if (elect_one()) {
           const int ky1 = min(a.kh, ky0 + kRowsPerStage);
           for (int ky = ky0; ky < ky1; ++ky) {
             const int grp = (ky >= gb1) + (ky >= gb2);
@@ -351,51 +380,29 @@ __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, 
             // two core matrices along K on both operands
             uint32_t ah = w_ahi + ky, al = w_alo + ky, av = w_avd + ky;
             uint32_t bh = w_ring + s * stage_w + (ky - ky0) * row_w, bl = bh + g.NB * 8, bf = bh + 2 * g.NB * 8;
-            mma_bf16(tg, ah, bh, f);
-            mma_bf16(t_corr, ah, bl, ky != 0);
-            mma_f16(t_corr, al, bf, 1u);
-            if (den_mma) {
-              mma_bf16(td, av, bh, f);
-              mma_bf16(td, av, bl, 1u);
-#pragma unroll 1
-              for (int ks = 1; ks < g.KS; ++ks) {
-                ah += a_ks;
-                al += a_ks;
-                av += a_ks;
-                bh += 16;
-                bl += 16;
-                bf += 16;
-                mma_bf16(tg, ah, bh, 1u);
-                mma_bf16(t_corr, ah, bl, 1u);
-                mma_f16(t_corr, al, bf, 1u);
-                mma_bf16(td, av, bh, 1u);
-                mma_bf16(td, av, bl, 1u);
-              }
-            } else {
-#pragma unroll 2
-              for (int ks = 1; ks < g.KS; ++ks) {
-                ah += a_ks;
-                al += a_ks;
-                bh += 16;
-                bl += 16;
-                bf += 16;
-                mma_bf16(tg, ah, bh, 1u);
-                mma_bf16(t_corr, ah, bl, 1u);
-                mma_f16(t_corr, al, bf, 1u);
-              }
+            switch (g.KS) {
+              case 4: issue_row<4>(tg, t_corr, td, ah, al, av, bh, bl, bf, a_ks, f, ky != 0, den_mma); break;
+              case 5: issue_row<5>(tg, t_corr, td, ah, al, av, bh, bl, bf, a_ks, f, ky != 0, den_mma); break;
+              case 6: issue_row<6>(tg, t_corr, td, ah, al, av, bh, bl, bf, a_ks, f, ky != 0, den_mma); break;
+              default: issue_row<7>(tg, t_corr, td, ah, al, av, bh, bl, bf, a_ks, f, ky != 0, den_mma); break;
             }
           }
           mma_commit(&b_empty[s]);  // the stage is free once these MMAs have read it
         }
-        if (!ok) break;
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (elect_one()) {
         mma_commit(&a_empty[b]);
         mma_commit(&acc_full[tb]);
       }
-      if (!ok) {
-        // MMAs already issued must finish before tensor memory is released
-        mma_commit(&drain_bar);
-        mbar_wait_bounded(&drain_bar, 0, err_word, kDevErrMmaTimeout);
-      }
+      __syncwarp();
+    }
+    if (!ok) {
+      // MMAs already issued must finish before tensor memory is released
+      if (elect_one()) mma_commit(&drain_bar);
+      __syncwarp();
+      mbar_wait_bounded(&drain_bar, 0, err_word, kDevErrMmaTimeout);
     }
   } else if (warp == 1) {
     // ========================================================= band producer
