@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kRThreads, 1) gauss_row_kernel(const GaussArgs
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(g_raw) + 1023) & ~uintptr_t(1023));
   const GaussGeom g = gauss_geom(a.k, 1);
   const RowPlan L = row_plan(g);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t npb = static_cast<uint32_t>((a.len + kRM - 1) / kRM);  // position blocks per line block
   const uint32_t nlb = static_cast<uint32_t>((a.lines + kRL - 1) / kRL);
   const int64_t total = static_cast<int64_t>(npb) * nlb * a.bands;
@@ -338,22 +338,25 @@ __global__ void __launch_bounds__(kRThreads, 1) gauss_row_kernel(const GaussArgs
 
   if (warp == 0) {
     // ========================================================= MMA issuer
-    if (lane == 0) {
-      const uint32_t ah0 = desc_lo(s_base + L.band, 128);
-      const uint32_t al0 = desc_lo(s_base + L.band + static_cast<uint32_t>(g.NB) * 128, 128);
-      const uint32_t k1 = (2 * L.lbo1) >> 4, k2 = (2 * L.lbo2) >> 4;  // one k-step: two core-matrix columns
-      int j = 0;
-      bool ok = true;
-      for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++j) {
-        const int b = j & 1;
-        ok = wait_or_abort(&b_full[b], (j >> 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
-        if (ok && j >= 2) ok = wait_or_abort(&acc_empty[b], ((j >> 1) - 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
-        if (!ok) break;
-        tc_fence_after();
-        uint32_t ah = ah0, al = al0;
-        uint32_t b1 = desc_lo(s_base + L.p1 + b * L.p1_bytes, L.lbo1);
-        uint32_t b2 = desc_lo(s_base + L.p2 + b * L.p2_bytes, L.lbo2);
-        const uint32_t d1 = tmem + b * kRAccStride, d2 = d1 + kRN1;
+    // (uniform warp, see elect_one: 12 uint16 bands of 10980^2 at k = 65 in
+    // 8479 us, both passes together; 8723 us with one lane in a branch)
+    const uint32_t ah0 = desc_lo(s_base + L.band, 128);
+    const uint32_t al0 = desc_lo(s_base + L.band + static_cast<uint32_t>(g.NB) * 128, 128);
+    const uint32_t k1 = (2 * L.lbo1) >> 4, k2 = (2 * L.lbo2) >> 4;  // one k-step: two core-matrix columns
+    int j = 0;
+    bool ok = true;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+      const int b = j & 1;
+      ok = wait_or_abort(&b_full[b], (j >> 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+      if (ok && j >= 2) ok = wait_or_abort(&acc_empty[b], ((j >> 1) - 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t ah = ah0, al = al0;
+      uint32_t b1 = desc_lo(s_base + L.p1 + b * L.p1_bytes, L.lbo1);
+      uint32_t b2 = desc_lo(s_base + L.p2 + b * L.p2_bytes, L.lbo2);
+      const uint32_t d1 = tmem + b * kRAccStride, d2 = d1 + kRN1;
+      if (elect_one()) {
 #pragma unroll 1
         for (int ks = 0; ks < g.KS; ++ks) {
           mma_f16_n(d1, ah, b1, kIdescN128, ks != 0);
@@ -367,11 +370,13 @@ __global__ void __launch_bounds__(kRThreads, 1) gauss_row_kernel(const GaussArgs
         }
         mma_commit(&acc_full[b]);
       }
-      if (!ok) {
-        // MMAs already issued must finish before tensor memory is released
-        mma_commit(&drain_bar);
-        mbar_wait_bounded(&drain_bar, 0, err_word, kDevErrMmaTimeout);
-      }
+      __syncwarp();
+    }
+    if (!ok) {
+      // MMAs already issued must finish before tensor memory is released
+      if (elect_one()) mma_commit(&drain_bar);
+      __syncwarp();
+      mbar_wait_bounded(&drain_bar, 0, err_word, kDevErrMmaTimeout);
     }
   } else {
     // ========================================================= converters + epilogue
@@ -615,7 +620,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gauss_col_kernel(const GaussArgs
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(g_raw) + 1023) & ~uintptr_t(1023));
   const GaussGeom g = gauss_geom(a.k, 2);
   const GaussPlan L = gauss_plan(g);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t npb = static_cast<uint32_t>((a.len + kGN - 1) / kGN);
   const uint32_t nlb = static_cast<uint32_t>((a.lines + kGL - 1) / kGL);
   const int64_t total = static_cast<int64_t>(npb) * nlb * a.bands;
@@ -646,22 +651,23 @@ __global__ void __launch_bounds__(kGThreads, 1) gauss_col_kernel(const GaussArgs
 
   if (warp == 0) {
     // ========================================================= MMA issuer
-    if (lane == 0) {
-      const uint32_t a_ks = (2 * L.lbo) >> 4;  // one k-step = two core matrices along K
-      const uint32_t bh0 = desc_lo(s_base + L.band, 128);
-      const uint32_t bl0 = desc_lo(s_base + L.band + static_cast<uint32_t>(g.NB) * 128, 128);
-      int j = 0;
-      bool ok = true;
-      for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++j) {
-        const int b = j & 1;
-        ok = wait_or_abort(&a_full[b], (j >> 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
-        if (ok && j >= 2) ok = wait_or_abort(&acc_empty[b], ((j >> 1) - 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
-        if (!ok) break;
-        tc_fence_after();
-        uint32_t ah = desc_lo(s_base + 2 * b * L.a_bytes, L.lbo);
-        uint32_t al = desc_lo(s_base + (2 * b + 1) * L.a_bytes, L.lbo);
-        uint32_t bh = bh0, bl = bl0;
-        const uint32_t t_hh = tmem + b * 2 * kGN, t_cr = t_hh + kGN;
+    const uint32_t a_ks = (2 * L.lbo) >> 4;  // one k-step = two core matrices along K
+    const uint32_t bh0 = desc_lo(s_base + L.band, 128);
+    const uint32_t bl0 = desc_lo(s_base + L.band + static_cast<uint32_t>(g.NB) * 128, 128);
+    int j = 0;
+    bool ok = true;
+    for (int64_t t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+      const int b = j & 1;
+      ok = wait_or_abort(&a_full[b], (j >> 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+      if (ok && j >= 2) ok = wait_or_abort(&acc_empty[b], ((j >> 1) - 1) & 1, &abort_flag, err_word, kDevErrMmaTimeout);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t ah = desc_lo(s_base + 2 * b * L.a_bytes, L.lbo);
+      uint32_t al = desc_lo(s_base + (2 * b + 1) * L.a_bytes, L.lbo);
+      uint32_t bh = bh0, bl = bl0;
+      const uint32_t t_hh = tmem + b * 2 * kGN, t_cr = t_hh + kGN;
+      if (elect_one()) {
 #pragma unroll 1
         for (int ks = 0; ks < g.KS; ++ks) {
           mma_f16(t_hh, ah, bh, ks != 0);
@@ -675,11 +681,13 @@ __global__ void __launch_bounds__(kGThreads, 1) gauss_col_kernel(const GaussArgs
         mma_commit(&a_empty[b]);
         mma_commit(&acc_full[b]);
       }
-      if (!ok) {
-        // MMAs already issued must finish before tensor memory is released
-        mma_commit(&drain_bar);
-        mbar_wait_bounded(&drain_bar, 0, err_word, kDevErrMmaTimeout);
-      }
+      __syncwarp();
+    }
+    if (!ok) {
+      // MMAs already issued must finish before tensor memory is released
+      if (elect_one()) mma_commit(&drain_bar);
+      __syncwarp();
+      mbar_wait_bounded(&drain_bar, 0, err_word, kDevErrMmaTimeout);
     }
   } else if (warp == 1) {
     // ========================================================= window copies
