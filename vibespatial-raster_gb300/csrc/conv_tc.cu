@@ -52,7 +52,7 @@
 //   warp 0      issues the tcgen05.mma chains of each tile
 //   warp 1      streams the Toeplitz bands, one kernel row per stage, into a
 //               shared-memory ring with cp.async.bulk
-//   warps 2..9  convert the next tile's window to BF16 hi/lo (+ validity) in
+//   warps 2..13 convert the next tile's window to BF16 hi/lo (+ validity) in
 //               the MMA layout straight from global memory, then run the
 //               previous tile's epilogue (tcgen05.ld, FP32 sums, stores)
 // The roles hand over through mbarriers: full/empty pairs for the A buffers
@@ -77,13 +77,19 @@ using namespace tc;
 
 constexpr int kM = kMmaM;          // output rows per tile (TMEM lanes, MMA M)
 constexpr int kTN = kMmaN;         // output columns per tile (MMA N)
-constexpr int kConvWarps = 8;      // warps 2..9
+// Converters (warps 2..13), kConvRows = 4 rows each at a time.  Conversion is
+// bound by latency, not by instructions, so more warps help while their
+// registers suffice: 31x31 at 8192^2 1191 us with 8 warps (168 registers, 6
+// rows), 1133 with 12 (128, a few spilled); 16 (96 registers) spill more and
+// were slower than 8.
+constexpr int kConvWarps = 12;
+constexpr int kEpiWarps = 8;       // of these, run the epilogue (4 lane quarters x 2 column halves)
 constexpr int kConvThreads = 32 * kConvWarps;
 constexpr int kThreadsTC = 64 + kConvThreads;
 constexpr int kMaxTCK = 41;
 constexpr int kMaxStages = 8;      // Toeplitz band ring depth (at most)
 constexpr int kRowsPerStage = 2;   // kernel rows per ring stage (one wait and one release per stage)
-constexpr int kConvRows = 6;       // window rows a converter warp loads per batch
+constexpr int kConvRows = 4;       // window rows a converter warp loads per batch
 
 struct TcGeom {
   int kh, kw;
@@ -319,7 +325,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, 
       mbar_init(&a_full[i], kConvThreads);
       mbar_init(&a_empty[i], 1);
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], kConvThreads);
+      mbar_init(&acc_empty[i], 32 * kEpiWarps);
     }
     for (int s = 0; s < L.nst; ++s) {
       mbar_init(&b_full[s], 1);
@@ -432,7 +438,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, 
     }
   } else {
     // ========================================================= converters + epilogue
-    const int cw = warp - 2;            // converter warp 0..7
+    const int cw = warp - 2;            // converter warp 0..11
     const int ct = tid - 64;            // converter thread
     const int quarter = warp & 3;       // the TMEM lane quarter this warp may read
     const int chalf = cw >> 2;          // epilogue: output columns 32*chalf .. +31
@@ -457,6 +463,7 @@ __global__ void __launch_bounds__(kThreadsTC, 1) conv_tc_kernel(const TcArgs a, 
         ok = false;
         return;
       }
+      if (cw >= kEpiWarps) return;  // converter-only warps
       tc_fence_after();
       const int64_t x0 = info_x0[slot], y0 = info_y0[slot], band = info_band[slot];
       const float* bsrc = a.src + band * a.band_stride;
