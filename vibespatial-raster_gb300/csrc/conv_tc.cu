@@ -48,9 +48,9 @@
 // poisoning) and +-inf are kept out of the GEMM; per-row bitmasks give
 // their window footprints: NaN, or the infinite sum the reference forms.
 //
-// Persistent CTA, one per SM, 6 warps with fixed roles:
+// Persistent CTA, one per SM, 14 warps with fixed roles:
 //   warp 0      issues the tcgen05.mma chains of each tile
-//   warp 1      streams the Toeplitz bands, one kernel row per stage, into a
+//   warp 1      streams the Toeplitz bands, two kernel rows per stage, into a
 //               shared-memory ring with cp.async.bulk
 //   warps 2..13 convert the next tile's window to BF16 hi/lo (+ validity) in
 //               the MMA layout straight from global memory, then run the
@@ -77,11 +77,11 @@ using namespace tc;
 
 constexpr int kM = kMmaM;          // output rows per tile (TMEM lanes, MMA M)
 constexpr int kTN = kMmaN;         // output columns per tile (MMA N)
-// Converters (warps 2..13), kConvRows = 4 rows each at a time.  Conversion is
-// bound by latency, not by instructions, so more warps help while their
-// registers suffice: 31x31 at 8192^2 1191 us with 8 warps (168 registers, 6
-// rows), 1133 with 12 (128, a few spilled); 16 (96 registers) spill more and
-// were slower than 8.
+// Converters (warps 2..13), kConvRows = 4 rows each at a time.  More warps hide
+// more of the conversion's latencies while their registers suffice: 31x31 at
+// 8192^2 1191 us with 8 warps (168 registers, 6 rows), 1133 with 12 (128, a
+// few spilled).  16 (96 registers) were slower than 8, 1431 against 1396,
+// measured before the rows went through the phases together.
 constexpr int kConvWarps = 12;
 constexpr int kEpiWarps = 8;       // of these, run the epilogue (4 lane quarters x 2 column halves)
 constexpr int kConvThreads = 32 * kConvWarps;
