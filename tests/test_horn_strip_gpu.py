@@ -72,3 +72,18 @@ def test_odd_rows_equal_padded_rows(vsr, nodata, mode):
         got.append([t[:, :w].cpu().numpy() for t in (s, a, hs)])
     for x, y in zip(*got):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("shape", [(3, 126), (66, 127), (130, 253), (257, 505)])
+@pytest.mark.parametrize("dtype", [np.uint8, np.int16, np.uint16])
+def test_integer_strips_equal_generic(vsr, dtype, shape):
+    """The same whole elevations as 8/16-bit (strips) and as int32 (one thread per pixel):
+    exact gradients, so every output is equal bit for bit."""
+    rng = np.random.default_rng(shape[0])
+    d = _dem(dtype, shape, rng)
+    d[rng.random(shape) < 0.01] = 9
+    for nd in (9, None):
+        a = vsr.raster_terrain(vsr.from_numpy(d, nodata=nd, affine=AFF))
+        b = vsr.raster_terrain(vsr.from_numpy(d.astype(np.int32), nodata=nd, affine=AFF))
+        for k in ("slope", "aspect", "hillshade"):
+            np.testing.assert_array_equal(a[k].to_numpy(), b[k].to_numpy())

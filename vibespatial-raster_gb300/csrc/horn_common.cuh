@@ -140,6 +140,22 @@ __device__ __forceinline__ float2 atan_poly_deg2(float2 t) {
   return mul2(t, p);
 }
 
+// 45 - atan(t) in degrees, rounded once at the end: what the scalar form's
+// ``45.0f - atan_poly_deg(t)`` compiles to (the last product and the
+// subtraction contracted).  The negated coefficients round alike.
+__device__ __forceinline__ float2 atan_rest_deg2(float2 t) {
+  const float2 u = mul2(t, t);
+  float2 p = f2(0.232309317f);
+  p = fma2(p, u, f2(-1.2526542f));
+  p = fma2(p, u, f2(3.20353885f));
+  p = fma2(p, u, f2(-5.52457099f));
+  p = fma2(p, u, f2(7.96905727f));
+  p = fma2(p, u, f2(-11.4285402f));
+  p = fma2(p, u, f2(19.0966035f));
+  p = fma2(p, u, f2(-57.2957414f));
+  return fma2(t, p, f2(45.0f));
+}
+
 // Slope in degrees from s = p^2 + q^2.  With rs = 1/sqrt(s) and r = s rs,
 // t = min(r, 1/r) = min(s rs, rs) and a = atan(t); the result is a for
 // s <= 1 and 90 - a above: 45 - (45 - a) or 45 + (45 - a), the sign taken
@@ -151,13 +167,16 @@ __device__ __forceinline__ float slope_deg(float s) {
   return 45.0f + copysignf(45.0f - a, s - 1.0f);
 }
 
+// FUSED: 45 - a rounded once, as in the scalar form.
+template <bool FUSED = false>
 __device__ __forceinline__ float2 slope_deg2(float2 s) {
   const float2 sp = add2(s, f2(1e-30f));
   const float2 rs = make_float2(rsqrt_approx(sp.x), rsqrt_approx(sp.y));
   const float2 r = mul2(s, rs);
   const float2 t = make_float2(fminf(r.x, rs.x), fminf(r.y, rs.y));
-  const float2 a = atan_poly_deg2(t);
-  const float2 d = fma2(a, f2(-1.0f), f2(45.0f));
+  float2 d;
+  if constexpr (FUSED) d = atan_rest_deg2(t);
+  else d = fma2(atan_poly_deg2(t), f2(-1.0f), f2(45.0f));
   return add2(f2(45.0f), copysign2(d, add2(s, f2(-1.0f))));
 }
 
@@ -180,13 +199,17 @@ __device__ __forceinline__ float aspect_deg(float p, float q) {
   return (270.0f - th) - copysignf(180.0f, 90.0f - th);
 }
 
+template <bool FUSED = false>
 __device__ __forceinline__ float2 aspect_deg2(float2 p, float2 q) {
   const float ap0 = fabsf(p.x), aq0 = fabsf(q.x), ap1 = fabsf(p.y), aq1 = fabsf(q.y);
   const float2 mn = make_float2(fmin_nan(ap0, aq0), fmin_nan(ap1, aq1));
   const float2 mx = add2(make_float2(fmax_nan(ap0, aq0), fmax_nan(ap1, aq1)), f2(1e-30f));
-  const float2 a0 = atan_poly_deg2(mul2(mn, make_float2(rcp_approx(mx.x), rcp_approx(mx.y))));
+  const float2 t = mul2(mn, make_float2(rcp_approx(mx.x), rcp_approx(mx.y)));
+  float2 d;
+  if constexpr (FUSED) d = atan_rest_deg2(t);
+  else d = fma2(atan_poly_deg2(t), f2(-1.0f), f2(45.0f));
   const float2 dpq = make_float2(ap0 - aq0, ap1 - aq1);
-  const float2 a1 = fma2(copysign2(fma2(a0, f2(-1.0f), f2(45.0f)), dpq), f2(-1.0f), f2(45.0f));
+  const float2 a1 = fma2(copysign2(d, dpq), f2(-1.0f), f2(45.0f));
   const float2 a2 = fma2(copysign2(fma2(a1, f2(-1.0f), f2(90.0f)), p), f2(-1.0f), f2(90.0f));
   const float2 th = make_float2(copysignf(a2.x, -q.x), copysignf(a2.y, -q.y));
   const float2 e = fma2(th, f2(-1.0f), f2(270.0f));
