@@ -95,10 +95,8 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
   // of the lane's columns (4 bits), each thread reading only its own
   __shared__ float4 wring[K][32];
   __shared__ uint32_t oring[K][32];
-  __shared__ float gtab[2 * K];  // the weights twice over, for a ring that starts anywhere
   auto g_at = [&](int t) { return a.g[t < R ? R - t : t - R]; };
   const int lane = threadIdx.x;
-  for (int t = lane; t < 2 * K; t += 32) gtab[t] = a.g[abs((t < K ? t : t - K) - R)];
   const int64_t xw = static_cast<int64_t>(blockIdx.x) * G::kCols - 4 * G::HL;
   const int64_t xs = xw + 4 * lane, ys = static_cast<int64_t>(blockIdx.y) * a.strip;
   const int nout = static_cast<int>(a.H - ys < a.strip ? a.H - ys : static_cast<int64_t>(a.strip));
@@ -193,13 +191,14 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
       wring[slot][lane] = in ? make_float4(w[0], w[1], w[2], w[3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       oring[slot][lane] = ok;
       slot = slot + 1 == K ? 0 : slot + 1;
-      // slot s holds the row of weight (s - slot) mod K
+      // tap t's row is in slot (slot + t) mod K; taps in ascending order, as in
+      // the numerator: rounding errors common to both sums cancel in the quotient
       float2 d0 = make_float2(0.0f, 0.0f), d1 = d0;
-      const float* gs = gtab + K - slot;
 #pragma unroll
-      for (int s = 0; s < K; ++s) {
-        const float4 x = wring[s][lane];
-        const float2 gt = make_float2(gs[s], gs[s]);
+      for (int t = 0; t < K; ++t) {
+        const int s = slot + t;
+        const float4 x = wring[s >= K ? s - K : s][lane];
+        const float2 gt = make_float2(g_at(t), g_at(t));
         d0 = __ffma2_rn(gt, make_float2(x.x, x.y), d0);
         d1 = __ffma2_rn(gt, make_float2(x.z, x.w), d1);
       }
@@ -210,11 +209,14 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
       w4[2] = d1.x;
       w4[3] = d1.y;
     } else if (i - 2 * R < r0 || i >= r1) {  // rows outside: only those inside weigh
-      float cs = 0.0f;
 #pragma unroll
-      for (int t = 0; t < K; ++t) cs += i - 2 * R + t >= r0 && i - 2 * R + t < r1 ? g_at(t) : 0.0f;
+      for (int c = 0; c < 4; ++c) w4[c] = 0.0f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) w4[c] = rd[c] * cs;
+      for (int t = 0; t < K; ++t) {
+        const float gt = i - 2 * R + t >= r0 && i - 2 * R + t < r1 ? g_at(t) : 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w4[c] = fmaf(gt, rd[c], w4[c]);
+      }
     } else {
 #pragma unroll
       for (int c = 0; c < 4; ++c) w4[c] = wd[c];
