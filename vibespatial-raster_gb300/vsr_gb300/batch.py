@@ -180,8 +180,9 @@ class PerTileGraph:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
             per_tile_launches(rasters, sigma=sigma, kernel_size=kernel_size, outs=self.outs)
-        # per tile: the Horn kernel, the Gaussian tap build and the separable Gaussian
-        self.launches = 3 * len(rasters)
+        # per tile: the Horn kernel and the separable Gaussian, which has a
+        # kernel of its own for the tap build outside 3..17 taps
+        self.launches = (2 if 3 <= kernel_size <= 17 else 3) * len(rasters)
 
     def replay(self):
         self.graph.replay()
