@@ -817,7 +817,7 @@ def leg_derivatives(args, dev, gpu) -> dict:
         "value": px / (ms * 1e-3) / 1e9, "unit": UNIT, "ms_per_step": ms, "steps": n, "gpu_launches": 1,
         "l2": "1 GiB in + 6 GiB out per step exceed L2; no flush",
         "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
-                     "peak_source": src, "kernel": "terrain_deriv_kernel<float>", "bytes_per_px": 28},
+                     "peak_source": src, "kernel": "terrain_strip<float>", "bytes_per_px": 28},
         "cpu_baseline": {"value": 1.0 / cpu_s / 1e9, "unit": UNIT, "cores": 1, "kind": "port",
                          "sample": "512 x 16384 rows of the same DEM, reference float64 TRI, TPI, curvature "
                                    "(3 calls), 1 thread"},
@@ -865,7 +865,7 @@ def leg_focal_stats(args, dev, gpu) -> dict:
         "l2": "241 MB in + 482 MB out per call exceed L2; no flush",
         "roofline": {"bound": "hbm", "achieved": 6 * px / (ms * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                      "frac": 6 * px / (ms * 1e-3) / 1e9 / hbm, "peak_source": src,
-                     "kernel": "focal_stat_kernel<int, std>", "bytes_per_px": 6},
+                     "kernel": "fs_strip_std", "bytes_per_px": 6},
         "cpu_baseline": {"value": per["std"]["cpu_gpix_s"], "unit": UNIT, "cores": 1, "kind": "port",
                          "sample": "256^2 crop (3-px halo), reference CPU focal statistic (the oracle's "
                                    "sliding-window restatement), 1 thread, per statistic in 'stats'"},

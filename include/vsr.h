@@ -169,9 +169,11 @@ VSR_API int vsr_horn_fused_bands(const void* dem, int dtype, int bands, int64_t 
  * border pixels and pixels whose window touches nodata get ``nodata_out``
  * (the reference writes the raster's nodata, else -9999).  Outputs of
  * ``out_dtype`` (the reference returns float64), row pitch ``out_pitch``; any
- * of tri / tpi / curvature may be NULL.  8/16-bit and float32 DEMs are
- * evaluated in double-float FP32 (error-free differences, compensated sums:
- * ~44 significant bits), int32 and float64 DEMs in FP64.
+ * of tri / tpi / curvature may be NULL.  8/16-bit DEMs, and float32 DEMs where
+ * the values of three rows share a unit, are evaluated in integers (TRI and
+ * TPI exact, the curvature a 96-bit product rounded once); other float32
+ * windows in double-float FP32 (error-free differences, compensated sums: ~44
+ * significant bits), int32 and float64 DEMs in FP64.
  */
 VSR_API int vsr_terrain_derivatives(const void* dem, int dtype, int64_t height, int64_t width, int64_t pitch,
                                     double cell_x, double cell_y, double nodata, int nodata_kind,
@@ -196,10 +198,13 @@ VSR_API int vsr_terrain_derivatives_bands(const void* dem, int dtype, int bands,
  * weights_host : kh*kw float64 row-major weights in HOST memory
  * precision    : VSR_PREC_*
  * workspace    : device scratch of vsr_convolve_workspace_size() bytes,
- *                256-byte aligned.  The host weights are copied into it with
- *                cudaMemcpyAsync on ``stream`` (so the call returns after the
- *                host copy has been staged) and turned into the kernel's
- *                operand images there by a small float64 prep kernel.
+ *                256-byte aligned.  Odd square kernels of 3 to 13 on 8/16-bit
+ *                and float32 rasters pass the weights as kernel arguments and
+ *                leave the workspace (still checked) untouched.  Otherwise the
+ *                host weights are copied into it with cudaMemcpyAsync on
+ *                ``stream`` (so the call returns after the host copy has been
+ *                staged) and turned into the kernel's operand images there by a
+ *                small float64 prep kernel.
  */
 VSR_API size_t vsr_convolve_workspace_size(int kh, int kw, int precision);
 VSR_API int vsr_convolve(const void* src, int dtype, int64_t height, int64_t width, int64_t pitch,
@@ -231,16 +236,17 @@ VSR_API int vsr_convolve_bands(const void* src, int dtype, int bands, int64_t ba
  * every scratch byte it reads); calls whose kernels overlap on the GPU (e.g.
  * on two streams at once) race on it.  No cudaMalloc, cudaFree or allocating
  * library routine is called.  ``weights_host`` is staged into the scratch
- * with cudaMemcpyAsync on ``stream``, as in vsr_convolve. */
+ * with cudaMemcpyAsync on ``stream`` where vsr_convolve does so. */
 VSR_API int vsr_convolve_noalloc(const void* src, int dtype, int64_t height, int64_t width, int64_t pitch,
                          const double* weights_host, int kh, int kw, double nodata, int nodata_kind,
                          void* dst, int out_dtype, int64_t out_pitch, int precision, void* stream);
 
 /* ---- Gaussian filter -----------------------------------------------------
  * Replaces raster_gaussian_filter (algebra.py:2120-2154): weights built in
- * float64 on the device (g_i = exp(-0.5 (i - k/2)^2 / sigma^2)); the filter is
- * evaluated separably (row pass held in shared memory, then the column pass),
- * which equals the reference's dense k x k normalised correlation with
+ * float64 (g_i = exp(-0.5 (i - k/2)^2 / sigma^2)), on the host for 3 to 17
+ * taps on 8/16-bit and float32 rasters (kernel arguments; the workspace is
+ * checked and not used), on the device otherwise; the filter is evaluated
+ * separably (row pass, then column pass), which equals the reference's dense k x k normalised correlation with
  * weights outer(g, g) / sum exactly in real arithmetic, nodata and borders
  * included.  kernel_size <= 0 selects the default 2*ceil(3 sigma)+1; even
  * sizes are bumped to odd.  Same output rule as vsr_convolve.
@@ -308,9 +314,11 @@ VSR_API int vsr_focal_mean_bands(const void* src, int dtype, int bands, int64_t 
  *   VSR_STAT_MEAN        as vsr_focal_mean;
  *   VSR_STAT_STD         population standard deviation of the valid
  *                        (non-nodata, non-NaN) taps, 0.0 for an empty window;
- *                        exact integer sums for 8/16-bit rasters (a VSR_F32
- *                        output is sqrt(n^2 var)/n rounded once to float32),
- *                        two passes in float64 otherwise;
+ *                        exact integer sums and sqrt(n^2 var)/n formed in
+ *                        integers (within 0.52 ulp of float64) for 8/16-bit
+ *                        rasters and for float32 ones where a strip's values
+ *                        fit one unit, up to radius 7; two passes in float64
+ *                        otherwise;
  *   VSR_STAT_RANGE       max - min of the valid taps;
  *   VSR_STAT_VARIETY     number of distinct valid values, 0 for an empty
  *                        window (no cap; the reference GPU kernel stops at 49).
