@@ -55,9 +55,14 @@ class RasterDeviceState:
     nodata_mask: object | None = None
 
 
-_TORCH_OF: dict = {}  # np.dtype -> torch.dtype, built on first use
-_NP_OF: dict = {}     # torch.dtype -> np.dtype
-_NAME_OF: dict = {}   # np.dtype -> str (numpy forms it in Python on each call)
+@dataclass(frozen=True)
+class _DtypeTables:
+    torch_of: dict  # np.dtype -> torch.dtype
+    np_of: dict     # torch.dtype -> np.dtype
+    name_of: dict   # np.dtype -> str (numpy forms it in Python on each call)
+
+
+_TABLES: _DtypeTables | None = None
 
 
 def _torch():
@@ -66,25 +71,29 @@ def _torch():
     return torch
 
 
-def _dtype_tables() -> None:
-    torch = _torch()
-    names = ("uint8", "int8", "int16", "uint16", "int32", "uint32", "int64", "float16", "float32", "float64", "bool")
-    table = {np.dtype(n): getattr(torch, n) for n in names}
-    _NP_OF.update({t: n for n, t in table.items()})
-    _NAME_OF.update({n: str(n) for n in table})
-    _TORCH_OF.update(table)  # in one step: another thread sees none or all
+def _dtype_tables() -> _DtypeTables:
+    """The tables, built on first use (torch is imported late).
+
+    Published in one assignment when they are complete: threads that arrive
+    meanwhile build the same tables again and never see a part of them.
+    """
+    global _TABLES
+    tables = _TABLES
+    if tables is None:
+        torch = _torch()
+        names = ("uint8", "int8", "int16", "uint16", "int32", "uint32", "int64", "float16", "float32", "float64",
+                 "bool")
+        torch_of = {np.dtype(n): getattr(torch, n) for n in names}
+        tables = _TABLES = _DtypeTables(torch_of, {t: n for n, t in torch_of.items()}, {n: str(n) for n in torch_of})
+    return tables
 
 
 def torch_dtype(np_dtype):
-    if not _TORCH_OF:
-        _dtype_tables()
-    return _TORCH_OF[np.dtype(np_dtype)]
+    return _dtype_tables().torch_of[np.dtype(np_dtype)]
 
 
 def numpy_dtype(t_dtype) -> np.dtype:
-    if not _NP_OF:
-        _dtype_tables()
-    return _NP_OF[t_dtype]
+    return _dtype_tables().np_of[t_dtype]
 
 
 def _host_to_device(host: np.ndarray):
@@ -407,7 +416,7 @@ def from_device(device_data, *, nodata=None, affine=(1.0, 0.0, 0.0, 0.0, -1.0, 0
         device_state=RasterDeviceState(data=t),
         _host_materialized=False,
         diagnostics=[
-            diagnostic_event(RasterDiagnosticKind.CREATED, f"from_device shape={shape} dtype={_NAME_OF[np_dt]}",
+            diagnostic_event(RasterDiagnosticKind.CREATED, f"from_device shape={shape} dtype={_dtype_tables().name_of[np_dt]}",
                              Residency.DEVICE)
         ],
     )
