@@ -6,6 +6,11 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
+import pytest
+
+from vsr_gb300 import buffers
+
 PKG = Path(__file__).resolve().parents[1] / "vibespatial-raster_gb300"
 
 # every trial starts from a freshly executed module, as a process's first use does
@@ -35,3 +40,18 @@ print(len(errors), errors[:3])
 def test_first_use_from_several_threads():
     out = subprocess.run([sys.executable, "-c", FIRST_USE], cwd=PKG, capture_output=True, text=True, check=True).stdout
     assert out.startswith("0 "), out
+
+
+def test_unfetched_pixels_cannot_be_written(monkeypatch):
+    """``data`` of a raster on the device is a placeholder that all such rasters share."""
+    import torch
+
+    monkeypatch.setattr(buffers, "as_device_tensor", lambda t: t)
+    a, b = (buffers.from_device(torch.zeros(shape)) for shape in ((4, 5), (2, 4, 5)))
+    assert a.data.shape == (4, 5) and b.data.dtype == np.float32 and b.data.nbytes == 160
+    with pytest.raises(ValueError):
+        a.data[1, 2] = 7.0
+    assert not b.data.any()
+    got = a.to_numpy()  # fetched: the raster's own buffer
+    got[1, 2] = 7.0
+    assert a.data[1, 2] == 7.0 and not b.to_numpy().any()

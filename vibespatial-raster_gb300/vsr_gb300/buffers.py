@@ -383,14 +383,15 @@ def as_device_tensor(device_data):
     return t
 
 
-_HOLD = bytearray(16)  # one element of any dtype
+_HOLD = bytes(16)  # one element of any dtype; immutable, so arrays over it are read-only
 
 
 def _host_placeholder(shape: tuple, dtype: np.dtype) -> np.ndarray:
     """Host array of ``shape`` for a raster whose pixels are on the device only.
 
-    Every element is the same 16 bytes (stride 0): shape, dtype and nbytes read
-    as those of the pixels, which ``to_numpy`` fetches.  Reserving host memory
+    Every element is the same 16 bytes (stride 0), shared by all such rasters:
+    shape, dtype and nbytes read as those of the pixels, which ``to_numpy``
+    fetches; writing raises, as it would be lost.  Reserving host memory
     of the raster's size instead cost 67 us per result (map and unmap; 4096^2
     and larger), more than most of the kernels take.
     """
