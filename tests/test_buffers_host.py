@@ -55,3 +55,11 @@ def test_unfetched_pixels_cannot_be_written(monkeypatch):
     got = a.to_numpy()  # fetched: the raster's own buffer
     got[1, 2] = 7.0
     assert a.data[1, 2] == 7.0 and not b.to_numpy().any()
+
+
+def test_events_built_without_init_are_whole():
+    kind, where = buffers.RasterDiagnosticKind.RUNTIME, buffers.Residency.DEVICE
+    for given in ({}, {"visible_to_user": True, "elapsed_seconds": 0.5}):
+        made, ref = (f(kind=kind, detail="d", residency=where, **given)
+                     for f in (buffers.diagnostic_event, buffers.RasterDiagnosticEvent))
+        assert made == ref and vars(made) == vars(ref)

@@ -142,7 +142,8 @@ def _shared_layout(*tensors) -> tuple[int, int]:
 
 
 def _record(result: OwnedRasterArray, detail: str, elapsed: float = 0.0) -> OwnedRasterArray:
-    result.diagnostics.append(diagnostic_event(RasterDiagnosticKind.RUNTIME, detail, Residency.DEVICE, True, elapsed))
+    result.diagnostics.append(diagnostic_event(RasterDiagnosticKind.RUNTIME, detail, Residency.DEVICE,
+                                               visible_to_user=True, elapsed_seconds=elapsed))
     return result
 
 

@@ -14,7 +14,7 @@ from __future__ import annotations
 import time
 import warnings
 from collections.abc import Sequence
-from dataclasses import dataclass, field
+from dataclasses import MISSING, dataclass, field, fields
 from enum import StrEnum
 
 import numpy as np
@@ -39,11 +39,13 @@ class RasterDiagnosticEvent:
     bytes_transferred: int = 0
 
 
-def diagnostic_event(kind, detail, residency, visible_to_user=False, elapsed_seconds=0.0) -> RasterDiagnosticEvent:
+_EVENT_DEFAULTS = {f.name: f.default for f in fields(RasterDiagnosticEvent) if f.default is not MISSING}
+
+
+def diagnostic_event(kind, detail, residency, **given) -> RasterDiagnosticEvent:
     """A RasterDiagnosticEvent without the per-field setattr of a frozen dataclass's __init__ (two per call)."""
     ev = object.__new__(RasterDiagnosticEvent)
-    ev.__dict__.update(kind=kind, detail=detail, residency=residency, visible_to_user=visible_to_user,
-                       elapsed_seconds=elapsed_seconds, bytes_transferred=0)
+    ev.__dict__.update(_EVENT_DEFAULTS, kind=kind, detail=detail, residency=residency, **given)
     return ev
 
 
