@@ -110,11 +110,11 @@ __global__ void __launch_bounds__(32) conv_warp(const __grid_constant__ CwArgs a
 #pragma unroll
     for (int c = 0; c < 4; ++c) wd[c] = d[c];
   }
-  bool odd = false;  // a weight sum whose reciprocal is not normal
+  bool odd = false;  // a weight sum whose reciprocal or quotients (numerators from 1e-30) may not be normal
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    wr[c] = strip_recip(wd[c]);
-    odd |= !(wd[c] > 1.0e-30f && wd[c] < 1.0e30f);
+    wr[c] = vsr_div_recip(wd[c]);
+    odd |= !(wd[c] > 1.0e-30f && wd[c] < 1.0e6f);
   }
   RowRing<T, kCwDepth> in_rows;
   in_rows.start(rows, src + (ys - R) * a.pitch + xw, a.pitch, xw, a.W, r0, r1, a.vin);
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(32) conv_warp(const __grid_constant__ CwArgs a
         }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          bad |= !(d[c] > 1.0e-30f && d[c] < 1.0e30f);
-          q[c] = strip_quot(done[c], d[c], strip_recip(d[c]), bad);
+          bad |= !(d[c] > 1.0e-30f && d[c] < 1.0e6f);
+          q[c] = strip_quot(done[c], d[c], vsr_div_recip(d[c]), bad);
         }
       } else {
 #pragma unroll

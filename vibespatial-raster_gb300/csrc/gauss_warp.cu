@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
       wd[c] = g_at(0) * rd[c];
 #pragma unroll
       for (int t = 1; t < K; ++t) wd[c] = fmaf(g_at(t), rd[c], wd[c]);
-      wr[c] = strip_recip(wd[c]);
+      wr[c] = vsr_div_recip(wd[c]);
     }
   }
   RowRing<T, kGwDepth> in_rows;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(32) gauss_warp(const __grid_constant__ GwArgs 
       float q[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        r4[c] = whole ? wr[c] : strip_recip(w4[c]);
+        r4[c] = whole ? wr[c] : vsr_div_recip(w4[c]);
         bad |= !(w4[c] > 1.0e-30f);
         q[c] = strip_quot(n4[c], w4[c], r4[c], bad);
       }
