@@ -111,38 +111,22 @@ __device__ __forceinline__ float2 copysign2(float2 mag, float2 sgn) {
 }
 
 // ------------------------------------------------------ angle arithmetic --
-// Degree-valued arctangent on t in [0, 1]: t * P(t^2), P the degree-7
-// minimax polynomial fitted by csrc/fit_atan.py (max error 2.1e-6 deg in
-// float64, 7.6e-6 deg evaluated in float32).
-__device__ __forceinline__ float atan_poly_deg(float t) {
+// 45 - atan(t) in degrees on t in [0, 1], rounded once at the end: fma(t, -P(t^2),
+// 45), P the degree-7 minimax polynomial fitted by csrc/fit_atan.py (t P: max
+// error 2.1e-6 deg in float64, 7.6e-6 deg evaluated in float32).
+__device__ __forceinline__ float atan_rest_deg(float t) {
   const float u = t * t;
-  float p = -0.232309317f;
-  p = fmaf(p, u, 1.2526542f);
-  p = fmaf(p, u, -3.20353885f);
-  p = fmaf(p, u, 5.52457099f);
-  p = fmaf(p, u, -7.96905727f);
-  p = fmaf(p, u, 11.4285402f);
-  p = fmaf(p, u, -19.0966035f);
-  p = fmaf(p, u, 57.2957414f);
-  return t * p;
+  float p = 0.232309317f;
+  p = fmaf(p, u, -1.2526542f);
+  p = fmaf(p, u, 3.20353885f);
+  p = fmaf(p, u, -5.52457099f);
+  p = fmaf(p, u, 7.96905727f);
+  p = fmaf(p, u, -11.4285402f);
+  p = fmaf(p, u, 19.0966035f);
+  p = fmaf(p, u, -57.2957414f);
+  return fmaf(t, p, 45.0f);
 }
 
-__device__ __forceinline__ float2 atan_poly_deg2(float2 t) {
-  const float2 u = mul2(t, t);
-  float2 p = f2(-0.232309317f);
-  p = fma2(p, u, f2(1.2526542f));
-  p = fma2(p, u, f2(-3.20353885f));
-  p = fma2(p, u, f2(5.52457099f));
-  p = fma2(p, u, f2(-7.96905727f));
-  p = fma2(p, u, f2(11.4285402f));
-  p = fma2(p, u, f2(-19.0966035f));
-  p = fma2(p, u, f2(57.2957414f));
-  return mul2(t, p);
-}
-
-// 45 - atan(t) in degrees, rounded once at the end: what the scalar form's
-// ``45.0f - atan_poly_deg(t)`` compiles to (the last product and the
-// subtraction contracted).  The negated coefficients round alike.
 __device__ __forceinline__ float2 atan_rest_deg2(float2 t) {
   const float2 u = mul2(t, t);
   float2 p = f2(0.232309317f);
@@ -163,28 +147,23 @@ __device__ __forceinline__ float2 atan_rest_deg2(float2 t) {
 __device__ __forceinline__ float slope_deg(float s) {
   const float rs = rsqrt_approx(s + 1e-30f);
   const float t = fminf(s * rs, rs);
-  const float a = atan_poly_deg(t);
-  return 45.0f + copysignf(45.0f - a, s - 1.0f);
+  return 45.0f + copysignf(atan_rest_deg(t), s - 1.0f);
 }
 
-// FUSED: 45 - a rounded once, as in the scalar form.
-template <bool FUSED = false>
 __device__ __forceinline__ float2 slope_deg2(float2 s) {
   const float2 sp = add2(s, f2(1e-30f));
   const float2 rs = make_float2(rsqrt_approx(sp.x), rsqrt_approx(sp.y));
   const float2 r = mul2(s, rs);
   const float2 t = make_float2(fminf(r.x, rs.x), fminf(r.y, rs.y));
-  float2 d;
-  if constexpr (FUSED) d = atan_rest_deg2(t);
-  else d = fma2(atan_poly_deg2(t), f2(-1.0f), f2(45.0f));
+  const float2 d = atan_rest_deg2(t);
   return add2(f2(45.0f), copysign2(d, add2(s, f2(-1.0f))));
 }
 
 // Aspect in compass degrees, (90 - theta) mod 360 with theta = atan2(-q, p)
 // in degrees, signed zeros as atan2 has them (flat gives exactly 90, the
 // axes exactly 0, 90, 180, 270):
-//   a0 = atan(min/max of |p|, |q|)                 in [0, 45]
-//   a1 = 45 - copysign(45 - a0, |p| - |q|)         angle from the x axis, [0, 90]
+//   d  = 45 - atan(min/max of |p|, |q|)            in [0, 45]
+//   a1 = 45 - copysign(d, |p| - |q|)               angle from the x axis, [0, 90]
 //   a2 = 90 - copysign(90 - a1, p)                 [0, 180]
 //   theta = copysign(a2, -q)
 //   aspect = (270 - theta) - copysign(180, 90 - theta)
@@ -192,22 +171,19 @@ __device__ __forceinline__ float2 slope_deg2(float2 s) {
 __device__ __forceinline__ float aspect_deg(float p, float q) {
   const float ap = fabsf(p), aq = fabsf(q);
   const float mn = fmin_nan(ap, aq), mx = fmax_nan(ap, aq);
-  const float a0 = atan_poly_deg(mn * rcp_approx(mx + 1e-30f));
-  const float a1 = 45.0f - copysignf(45.0f - a0, ap - aq);
+  const float d = atan_rest_deg(mn * rcp_approx(mx + 1e-30f));
+  const float a1 = 45.0f - copysignf(d, ap - aq);
   const float a2 = 90.0f - copysignf(90.0f - a1, p);
   const float th = copysignf(a2, -q);
   return (270.0f - th) - copysignf(180.0f, 90.0f - th);
 }
 
-template <bool FUSED = false>
 __device__ __forceinline__ float2 aspect_deg2(float2 p, float2 q) {
   const float ap0 = fabsf(p.x), aq0 = fabsf(q.x), ap1 = fabsf(p.y), aq1 = fabsf(q.y);
   const float2 mn = make_float2(fmin_nan(ap0, aq0), fmin_nan(ap1, aq1));
   const float2 mx = add2(make_float2(fmax_nan(ap0, aq0), fmax_nan(ap1, aq1)), f2(1e-30f));
   const float2 t = mul2(mn, make_float2(rcp_approx(mx.x), rcp_approx(mx.y)));
-  float2 d;
-  if constexpr (FUSED) d = atan_rest_deg2(t);
-  else d = fma2(atan_poly_deg2(t), f2(-1.0f), f2(45.0f));
+  const float2 d = atan_rest_deg2(t);
   const float2 dpq = make_float2(ap0 - aq0, ap1 - aq1);
   const float2 a1 = fma2(copysign2(d, dpq), f2(-1.0f), f2(45.0f));
   const float2 a2 = fma2(copysign2(fma2(a1, f2(-1.0f), f2(90.0f)), p), f2(-1.0f), f2(90.0f));

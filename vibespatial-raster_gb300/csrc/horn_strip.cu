@@ -5,11 +5,10 @@
 // lane's place j, so that every store instruction writes 32 adjacent outputs
 // whatever the rows' alignment; rows arrive through shared memory
 // (warp_strip.cuh) and the last three rows' windows stay in registers.  The
-// arithmetic is horn_common.cuh's, two pixels per packed instruction: integer
-// DEMs with the generic (scalar) kernel's results bit for bit, float32 DEMs
-// with the TMA kernel's, which rounds once more in the arctangents.  float64 outputs are the float
-// results widened by integer operations (a conversion would occupy the FP64
-// pipe, two operations per clock and SM).
+// arithmetic is horn_common.cuh's, two pixels per packed instruction: the
+// generic (scalar) kernel's results bit for bit, and the TMA kernel's.  float64
+// outputs are the float results widened by integer operations (a conversion
+// would occupy the FP64 pipe, two operations per clock and SM).
 //
 // Bound by instruction issue and, with float64 outputs, HBM (19 B/px for
 // 16-bit DEMs).
@@ -25,7 +24,7 @@ namespace {
 constexpr int kHsCols = 126;
 constexpr int kHsDepth = 6;  // rows in shared memory
 
-// The values at and beside a lane's 4 columns in one row, and their range.
+// The values at and beside a lane's 4 columns in one row, and the row's nodata.
 struct HsRow {
   float l[4], c[4], r[4];
   uint32_t nd[4], dil[4];  // nodata at / at or beside a column, a bit per lane
@@ -146,12 +145,12 @@ __global__ void __launch_bounds__(32) horn_strip(const T* __restrict__ src, cons
         const float2 q = mul2(make_float2(gy[k], gy[k + 1]), f2(P.inv8cy));
         const float2 s = fma2(p, p, mul2(q, q));
         if (slope) {
-          const float2 v = slope_deg2<!kFloat>(s);
+          const float2 v = slope_deg2(s);
           so[k] = v.x;
           so[k + 1] = v.y;
         }
         if (aspect) {
-          const float2 v = aspect_deg2<!kFloat>(p, q);
+          const float2 v = aspect_deg2(p, q);
           ao[k] = v.x;
           ao[k + 1] = v.y;
         }
