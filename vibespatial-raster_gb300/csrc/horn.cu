@@ -9,8 +9,8 @@
 //  * horn_f32_tma  -- float32 rasters with 16-byte aligned rows
 //    (horn_tma.cuh; instantiated in horn_tma_all.cu / horn_tma_sub.cu).
 //  * horn_strip    -- 8/16-bit rasters and other float32 ones (horn_strip.cu).
-//  * horn_generic  -- int32 and float64: one thread per pixel, clamped loads
-//    through L1.
+//  * horn_generic  -- int32 and float64, and what is too small for the strips:
+//    one thread per pixel, clamped loads through L1.
 #include <type_traits>
 
 #include "horn_common.cuh"
@@ -43,6 +43,12 @@ __device__ __forceinline__ PixelOut horn_pixel(float gx, float gy, const HornPar
   return o;
 }
 
+// Exact differences: small integers in float, wider types in double.
+template <typename T>
+struct DiffType { using type = float; };
+template <> struct DiffType<double> { using type = double; };
+template <> struct DiffType<int32_t> { using type = double; };
+
 template <typename O> __device__ __forceinline__ O nd_out(const HornParams& P);
 template <> __device__ __forceinline__ float nd_out<float>(const HornParams& P) { return P.nd_out_f; }
 template <> __device__ __forceinline__ double nd_out<double>(const HornParams& P) { return P.nd_out_d; }
@@ -51,7 +57,7 @@ template <typename T, typename O>
 __global__ void __launch_bounds__(256) horn_generic(const T* __restrict__ src, const HornParams P,
                                                     const NodataTest<T> nd, O* __restrict__ slope,
                                                     O* __restrict__ aspect, uint8_t* __restrict__ hs) {
-  using D = double;
+  using D = typename DiffType<T>::type;
   const int64_t x = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
   const int64_t y = static_cast<int64_t>(blockIdx.y) * 8 + threadIdx.y;
   if (x >= P.width || y >= P.height) return;
@@ -77,8 +83,13 @@ __global__ void __launch_bounds__(256) horn_generic(const T* __restrict__ src, c
     }
   }
   float gx, gy;
-  gx = static_cast<float>((v[0][2] - v[0][0]) + D(2) * (v[1][2] - v[1][0]) + (v[2][2] - v[2][0]));
-  gy = static_cast<float>((v[2][0] - v[0][0]) + D(2) * (v[2][1] - v[0][1]) + (v[2][2] - v[0][2]));
+  if constexpr (std::is_same<T, float>::value) {  // float differences may round
+    gx = grad_exact(v[0][0], v[0][2], v[1][0], v[1][2], v[2][0], v[2][2]);
+    gy = grad_exact(v[0][0], v[2][0], v[0][1], v[2][1], v[0][2], v[2][2]);
+  } else {
+    gx = static_cast<float>((v[0][2] - v[0][0]) + D(2) * (v[1][2] - v[1][0]) + (v[2][2] - v[2][0]));
+    gy = static_cast<float>((v[2][0] - v[0][0]) + D(2) * (v[2][1] - v[0][1]) + (v[2][2] - v[0][2]));
+  }
   const PixelOut o = horn_pixel(gx, gy, P, slope != nullptr, aspect != nullptr, hs != nullptr);
   const bool sa_nd = rule.sa_any && (rule.sa_center ? ctr : dil);
   if (slope) slope[y * P.out_pitch + x] = sa_nd ? nd_out<O>(P) : static_cast<O>(o.slope);
@@ -104,7 +115,11 @@ template <typename O>
 int dispatch_generic(int dtype, const void* src, const HornParams& P, double ndv, void* slope,
                      void* aspect, uint8_t* hs, cudaStream_t st) {
   switch (dtype) {
+    case VSR_F32: return launch_generic<float, O>(src, P, ndv, slope, aspect, hs, st);
     case VSR_F64: return launch_generic<double, O>(src, P, ndv, slope, aspect, hs, st);
+    case VSR_U8: return launch_generic<uint8_t, O>(src, P, ndv, slope, aspect, hs, st);
+    case VSR_I16: return launch_generic<int16_t, O>(src, P, ndv, slope, aspect, hs, st);
+    case VSR_U16: return launch_generic<uint16_t, O>(src, P, ndv, slope, aspect, hs, st);
     case VSR_I32: return launch_generic<int32_t, O>(src, P, ndv, slope, aspect, hs, st);
     default: return fail(VSR_ERR_INVALID_ARG, "unsupported dtype %d", dtype);
   }

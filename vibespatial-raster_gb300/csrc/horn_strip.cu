@@ -23,6 +23,14 @@ namespace {
 
 constexpr int kHsCols = 126;
 constexpr int kHsDepth = 6;  // rows in shared memory
+// Blocks per SM (strips of 8 rows) from which the strips are used.  With fewer,
+// a block's 10 rows one after the other take longer than one pixel per thread
+// (horn.cu).  us, pixels | strips: slope of int16 300^2 4.2 | 10.5, 1024^2 10.4
+// | 12.4, 1230^2 14.4 | 12.9; all three of int16 725^2 8.3 | 14.5, 1230^2 16.5 |
+// 17.3, 2048^2 39 | 36; float32 odd rows 300^2 4.2 | 10.6, 850^2 12.4 | 12.4,
+// 1024^2 16.4 | 12.4.
+template <typename T>
+constexpr int kHsFew = sizeof(T) < 4 ? 8 : 6;
 
 // The values at and beside a lane's 4 columns in one row, and the row's nodata.
 struct HsRow {
@@ -200,6 +208,7 @@ template <typename T, typename O>
 int launch_hs(const void* src, const HornParams& P, double ndv, void* slope, void* aspect, uint8_t* hs,
               cudaStream_t st) {
   const int64_t gx = (P.width + kHsCols - 1) / kHsCols;
+  if (gx * ((P.height + 7) / 8) * P.bands < kHsFew<T> * static_cast<int64_t>(sm_count())) return -1;
   int strip = 64;
   while (strip > 8 && gx * ((P.height + strip - 1) / strip) * P.bands < 32 * static_cast<int64_t>(sm_count())) strip /= 2;
   const int64_t gy = (P.height + strip - 1) / strip;
@@ -214,7 +223,7 @@ int launch_hs(const void* src, const HornParams& P, double ndv, void* slope, voi
 
 }  // namespace
 
-// -1: not a DEM this kernel takes.
+// -1: not a DEM this kernel takes, or too few strips.
 int run_horn_strip(int dtype, const void* src, const HornParams& P, double ndv, void* slope, void* aspect, bool f64,
                    uint8_t* hs, cudaStream_t st) {
   switch (dtype) {
