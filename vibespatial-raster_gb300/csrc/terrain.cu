@@ -26,9 +26,13 @@ namespace {
 constexpr int kDTW = 32, kDTH = 8;  // output tile: 32 x 8 pixels, one per thread
 constexpr int kDSW = kDTW + 2, kDSH = kDTH + 2;
 
+// One pixel per thread.  int32 and float64 DEMs in FP64 with the reference's
+// formulas; 8/16-bit and float32 DEMs of too few strips in the strips' integers
+// (and FP64 for the curvature) window by window.
 template <typename T>
 __global__ void __launch_bounds__(kDTW * kDTH) terrain_deriv_kernel(const T* __restrict__ src, const DerivParams P) {
-  using C = double;
+  using C = std::conditional_t<std::is_same<T, int32_t>::value || std::is_same<T, double>::value, double,
+                               std::conditional_t<std::is_same<T, float>::value, float, int32_t>>;
   __shared__ C tile[kDSH][kDSW + 1];
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kDTW + tx;
   const int64_t x0 = static_cast<int64_t>(blockIdx.x) * kDTW, y0 = static_cast<int64_t>(blockIdx.y) * kDTH;
@@ -43,7 +47,6 @@ __global__ void __launch_bounds__(kDTW * kDTH) terrain_deriv_kernel(const T* __r
   }
   __syncthreads();
   const int64_t x = x0 + tx, y = y0 + ty;
-  if (x >= P.W || y >= P.H) return;
   const int64_t o = static_cast<int64_t>(blockIdx.z) * P.out_band_stride + y * P.out_pitch + x;
   C z[9];
 #pragma unroll
@@ -57,16 +60,29 @@ __global__ void __launch_bounds__(kDTW * kDTH) terrain_deriv_kernel(const T* __r
 #pragma unroll
     for (int k = 0; k < 9; ++k) nd |= z[k] != z[k];
   }
+  WindowUnit unit{};
+  if constexpr (std::is_same<C, float>::value) {
+    // one size of integers per warp: what 32 bits hold, 64 hold as well
+    unit = window_unit(z);
+    if (nd) unit.size = kUnit32;
+    if (__any_sync(0xffffffffu, unit.size == kUnit64) && unit.size == kUnit32) unit.size = kUnit64;
+  }
+  if (x >= P.W || y >= P.H) return;
   if (nd) {
     if (P.tri) store_out(P.tri, P.out_dtype, o, P.nd_out);
     if (P.tpi) store_out(P.tpi, P.out_dtype, o, P.nd_out);
     if (P.curv) store_out(P.curv, P.out_dtype, o, P.nd_out);
     return;
   }
-  // FP64 DEMs and int32 DEMs: the reference's formulas in double
-  if (P.tri) store_out(P.tri, P.out_dtype, o, plain_tri(z));
-  if (P.tpi) store_out(P.tpi, P.out_dtype, o, plain_tpi(z));
-  if (P.curv) store_out(P.curv, P.out_dtype, o, plain_curv(z, P));
+  if constexpr (std::is_same<C, double>::value) {
+    if (P.tri) store_out(P.tri, P.out_dtype, o, plain_tri(z));
+    if (P.tpi) store_out(P.tpi, P.out_dtype, o, plain_tpi(z));
+    if (P.curv) store_out(P.curv, P.out_dtype, o, plain_curv(z, P));
+  } else if constexpr (std::is_same<C, float>::value) {
+    deriv_pixel(z, unit, o, P);
+  } else {
+    deriv_ints(z, 0, o, P);
+  }
 }
 
 template <typename T>
@@ -154,10 +170,19 @@ extern "C" int vsr_terrain_derivatives_bands(const void* dem, int dtype, int ban
   P.curv = curvature;
   P.out_dtype = out_dtype;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  P.kx = 100.0 / P.cx2;
+  P.ky = 100.0 / P.cy2;
   P.ck = curvature_factors(P.cx2, P.cy2);
-  if (dtype == VSR_I32) return launch_deriv<int32_t>(dem, P, bands, st);
-  if (dtype == VSR_F64) return launch_deriv<double>(dem, P, bands, st);
-  return run_terrain_strip(dem, dtype, P, bands, st);
+  const int rc = run_terrain_strip(dem, dtype, P, bands, st);
+  if (rc >= 0) return rc;
+  switch (dtype) {
+    case VSR_U8: return launch_deriv<uint8_t>(dem, P, bands, st);
+    case VSR_I16: return launch_deriv<int16_t>(dem, P, bands, st);
+    case VSR_U16: return launch_deriv<uint16_t>(dem, P, bands, st);
+    case VSR_I32: return launch_deriv<int32_t>(dem, P, bands, st);
+    case VSR_F32: return launch_deriv<float>(dem, P, bands, st);
+    default: return launch_deriv<double>(dem, P, bands, st);
+  }
 }
 
 extern "C" int vsr_terrain_derivatives(const void* dem, int dtype, int64_t height, int64_t width, int64_t pitch,

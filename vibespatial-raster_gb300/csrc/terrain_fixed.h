@@ -44,6 +44,20 @@ VSR_TF_FN uint32_t vsr_tf_shl(uint32_t hi, uint32_t lo, int z) {  // high word o
 #endif
 }
 
+// float64 bits of s 2^e, rounded to nearest (to even); |s| < 2^63 and a normal
+// result.  (A conversion would run on the narrow FP64 pipe.)
+VSR_TF_FN uint64_t vsr_wide_bits(int64_t s, int e) {
+  const uint64_t neg = (uint64_t)(s >> 63), m = ((uint64_t)s ^ neg) - neg;
+  const int w = (m >> 32) == 0u;  // a low word only
+  const uint32_t x0 = w ? (uint32_t)m : (uint32_t)(m >> 32), x1 = w ? 0u : (uint32_t)m;
+  const int z = vsr_tf_clz32(x0 | 1u);
+  const uint32_t f0 = vsr_tf_shl(x0, x1, z), f1 = x1 << z;  // the leading bit on top
+  const uint64_t mant = (uint64_t)(f0 >> 11) << 32 | vsr_tf_shl(f0, f1, 21);  // 53 bits
+  const uint64_t r = mant + (((f1 & 0x7ffu) + 0x3ffu + ((uint32_t)mant & 1u)) >> 11);  // (2^53 when it carries)
+  const uint32_t ex = (uint32_t)(1023 + 63 - 1 - z - (w ? 32 : 0) + e);
+  return x0 ? r + ((uint64_t)((ex << 20) | ((uint32_t)neg & 0x80000000u)) << 32) : 0u;
+}
+
 // float64 bits of -(a kx + b ky) 2^u; |a|, |b| < 2^29 and a normal result.
 // Without branches: lanes differ in sign and length.  A negative value is
 // taken as its ones' complement, one unit of 2^-s (2^-59 of a factor) off.

@@ -1,8 +1,9 @@
-// Terrain derivatives of one pixel (terrain.cu, terrain_strip.cu): the formulas
-// and the double-float arithmetic.
+// Terrain derivatives of one pixel (terrain.cu, terrain_strip.cu): the formulas,
+// the integer forms and the double-float arithmetic.
 //
-// GB300's FP64 rate is a small fraction of its FP32 rate, so windows of
-// 8/16-bit and float32 elevations that the integer forms do not take are
+// GB300's FP64 rate is a small fraction of its FP32 rate, so 8/16-bit and
+// float32 elevations are taken as integers in one unit per window (32 or 64
+// bits): TRI and TPI are exact and rounded once.  Windows that no unit holds are
 // evaluated in double-float FP32: every neighbour difference is formed
 // error-free (TwoDiff), sums are compensated (TwoSum) and products use FMA, so
 // results carry ~44 significant bits before the single conversion to the
@@ -30,8 +31,17 @@ struct DerivParams {
   float icx2_hi, icx2_lo, icy2_hi, icy2_lo;  // the same as float pairs
   void *tri, *tpi, *curv;
   int out_dtype;
-  vsr_curv_k ck;    // the curvature factors as integers (terrain_fixed.h)
+  double kx, ky;    // the curvature factors 100 / cx^2, 100 / cy^2
+  vsr_curv_k ck;    // the same as integers (terrain_fixed.h)
 };
+
+// Binades of the values of a 32-bit unit: |n| < 2^27, or 2^28 where no value is
+// negative; differences stay below 2^28, the sums of eight below 2^31.
+constexpr uint32_t kTdSpan = 4, kTdSpanPos = 5;
+// ... of a 64-bit unit: |n| < 2^58, the sums of eight differences below 2^62.
+constexpr uint32_t kTdSpanWide = 35;
+// Exponents of values whose scaled results are normal float64 numbers.
+constexpr uint32_t kTdExpMin = 64u, kTdExpMax = 190u;
 
 // ---- double-float helpers: value = hi + lo with |lo| <= ulp(hi)/2
 struct DF {
@@ -121,9 +131,87 @@ __device__ __forceinline__ C plain_curv(const C z[9], const DerivParams& P) {
   return C(-2) * (D + E) * C(100);
 }
 
-// One pixel of a float32-exact DEM from its window, in double-float where the
-// exact integers do not apply.
-__device__ __forceinline__ void deriv_pixel(const float z[9], int64_t o, const DerivParams& P) {
+// float64 bits of s 2^e, e20 = e 2^20: s + 2^31 as the low word of 2^52 + .,
+// one FP64 subtraction.
+__device__ __forceinline__ uint64_t scaled_bits(int32_t s, uint32_t e20) {
+  const double d = __hiloint2double(0x43300000, s ^ static_cast<int32_t>(0x80000000u)) -
+                   (4503599627370496.0 + 2147483648.0);
+  return static_cast<uint64_t>(__double_as_longlong(
+      __hiloint2double(__double2hiint(d) + static_cast<int32_t>(s ? e20 : 0u), __double2loint(d))));
+}
+template <typename B>
+__device__ __forceinline__ B out_bits(uint64_t b64) {
+  if constexpr (sizeof(B) == 8) return b64;
+  else return __float_as_uint(static_cast<float>(__longlong_as_double(static_cast<long long>(b64))));
+}
+
+// A finite float as an integer in units of 2^(e0 - 150), e0 its unit's lowest
+// exponent.
+__device__ __forceinline__ long long wide_int(float v, uint32_t e0) {
+  const uint32_t b = __float_as_uint(v);
+  const long long m = static_cast<long long>((b & 0x7fffffu) | 0x800000u) << ((((b >> 23) & 0xffu) - e0) & 63u);
+  return (b << 1) == 0u ? 0ll : (b >> 31 ? -m : m);
+}
+
+// Eight times TRI and TPI in the values' unit: exact.
+__device__ __forceinline__ int32_t abs_of(int32_t v) { return abs(v); }
+__device__ __forceinline__ long long abs_of(long long v) { return llabs(v); }
+template <typename N>
+__device__ __forceinline__ N tri8_of(N tl, N tc, N tr, N ml, N c, N mr, N bl, N bc, N br) {
+  return (abs_of(tl - c) + abs_of(tc - c)) + (abs_of(tr - c) + abs_of(ml - c)) + (abs_of(mr - c) + abs_of(bl - c)) +
+         (abs_of(bc - c) + abs_of(br - c));
+}
+template <typename N>
+__device__ __forceinline__ N tpi8_of(N tl, N tc, N tr, N ml, N c, N mr, N bl, N bc, N br) {
+  return 8 * c - ((tl + tc + tr) + (ml + mr) + (bl + bc + br));
+}
+
+// Curvature from the exact neighbour sums a and b as doubles: what the integer
+// product does not take (values of more binades, factors far apart).  Errors:
+// the factors', one rounding per product and sum, against five roundings of the
+// float64 formula.
+__device__ __forceinline__ uint64_t curv_bits_f64(uint64_t a, uint64_t b, const DerivParams& P) {
+  const double da = __longlong_as_double(static_cast<long long>(a)), db = __longlong_as_double(static_cast<long long>(b));
+  return static_cast<uint64_t>(__double_as_longlong(-fma(da, P.kx, db * P.ky)));
+}
+__device__ __forceinline__ uint64_t curv_bits_f64(int32_t a, int32_t b, int u, const DerivParams& P) {
+  return curv_bits_f64(vsr_int_scaled_bits(a, u), vsr_int_scaled_bits(b, u), P);
+}
+
+__device__ __forceinline__ void put_bits(void* base, int out_dtype, int64_t i, uint64_t b) {
+  if (out_dtype == VSR_F64) static_cast<uint64_t*>(base)[i] = b;
+  else static_cast<uint32_t*>(base)[i] = out_bits<uint32_t>(b);
+}
+
+// One pixel from its window's integers in units of 2^u.
+__device__ __forceinline__ void deriv_ints(const int32_t n[9], int u, int64_t o, const DerivParams& P) {
+  const uint32_t e20 = static_cast<uint32_t>(u - 3) << 20;
+  const int32_t a = n[3] + n[5] - 2 * n[4], b = n[1] + n[7] - 2 * n[4];
+  if (P.tri)
+    put_bits(P.tri, P.out_dtype, o, scaled_bits(tri8_of(n[0], n[1], n[2], n[3], n[4], n[5], n[6], n[7], n[8]), e20));
+  if (P.tpi)
+    put_bits(P.tpi, P.out_dtype, o, scaled_bits(tpi8_of(n[0], n[1], n[2], n[3], n[4], n[5], n[6], n[7], n[8]), e20));
+  if (P.curv)
+    put_bits(P.curv, P.out_dtype, o, P.ck.ok ? vsr_curv_bits(a, b, &P.ck, u) : curv_bits_f64(a, b, u, P));
+}
+__device__ __forceinline__ void deriv_ints(const long long n[9], int u, int64_t o, const DerivParams& P) {
+  if (P.tri)
+    put_bits(P.tri, P.out_dtype, o, vsr_wide_bits(tri8_of(n[0], n[1], n[2], n[3], n[4], n[5], n[6], n[7], n[8]), u - 3));
+  if (P.tpi)
+    put_bits(P.tpi, P.out_dtype, o, vsr_wide_bits(tpi8_of(n[0], n[1], n[2], n[3], n[4], n[5], n[6], n[7], n[8]), u - 3));
+  if (P.curv)
+    put_bits(P.curv, P.out_dtype, o,
+             curv_bits_f64(vsr_wide_bits(n[3] + n[5] - 2 * n[4], u), vsr_wide_bits(n[1] + n[7] - 2 * n[4], u), P));
+}
+
+// A pixel from a window that no unit holds (more than 35 binades, values of
+// extreme exponents, infinities, NaN): double-float, or integers without the
+// curvature where exponents are extreme but alike.
+struct Window {
+  float z[9];
+};
+static __device__ __noinline__ void deriv_df(const Window w, int64_t o, const DerivParams& P) {
+  const float* z = w.z;
   // finiteness of the values each formula reads: TRI and TPI all nine,
   // curvature the centre and its four edge neighbours
   bool f5 = true, f9;
@@ -194,7 +282,46 @@ __device__ __forceinline__ void deriv_pixel(const float z[9], int64_t o, const D
   }
 }
 
-// Derivatives of 8/16-bit and float32 DEMs (terrain_strip.cu).
+// The unit that holds a window, its lowest exponent and the integers' size.
+enum { kUnit32, kUnit64, kUnitNone };
+struct WindowUnit {
+  uint32_t e;
+  int size;
+};
+__device__ __forceinline__ WindowUnit window_unit(const float z[9]) {
+  uint32_t lo = 0xffffffffu, hi = 0u, sign = 0u;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const uint32_t b = __float_as_uint(z[k]), m = b & 0x7fffffffu;
+    lo = min(lo, m - 1u);  // zeros last
+    hi = max(hi, m);
+    sign |= m ? b : 0u;
+  }
+  const uint32_t eh = hi ? hi >> 23 : 127u, el = hi ? (lo + 1u) >> 23 : 127u;  // zeros only: any unit
+  if (el < kTdExpMin || eh > kTdExpMax || eh - el >= kTdSpanWide) return {el, kUnitNone};
+  return {el, eh - el < (sign >> 31 ? kTdSpan : kTdSpanPos) ? kUnit32 : kUnit64};
+}
+
+// One pixel of a float32 DEM from its window.
+__device__ __forceinline__ void deriv_pixel(const float z[9], WindowUnit w, int64_t o, const DerivParams& P) {
+  if (w.size == kUnit32) {
+    const float scale = __uint_as_float((277u - w.e) << 23);  // 2^(150 - e)
+    int32_t n[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) n[k] = __float2int_rn(z[k] * scale);
+    deriv_ints(n, static_cast<int>(w.e) - 150, o, P);
+  } else if (w.size == kUnit64) {
+    long long n[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) n[k] = wide_int(z[k], w.e);
+    deriv_ints(n, static_cast<int>(w.e) - 150, o, P);
+  } else {
+    deriv_df(Window{z[0], z[1], z[2], z[3], z[4], z[5], z[6], z[7], z[8]}, o, P);
+  }
+}
+
+// Derivatives of 8/16-bit and float32 DEMs (terrain_strip.cu); -1: too few
+// strips to fill the GPU.
 int run_terrain_strip(const void* dem, int dtype, const DerivParams& P, int bands, cudaStream_t st);
 
 }  // namespace vsr

@@ -3,9 +3,9 @@
 //
 // Semantics and formulas: terrain.cu.  Elevations that lie within four
 // binades of each other (five if none is negative) are integers below 2^27
-// (2^28) in one unit; TRI and TPI are
-// then exact integers (terrain_exact.h: the reference's float64 results bit for
-// bit) and the curvature is a fixed-point product (terrain_fixed.h).
+// (2^28) in one unit; TRI and TPI are then exact integers (the reference's
+// float64 results bit for bit) and the curvature is a fixed-point product
+// (terrain_fixed.h), or two FP64 products where its factors are far apart.
 //
 // A warp walks down 126 columns (128 with the halo), column 32 j + lane in a
 // lane's place j, so that every store instruction writes 256 contiguous bytes
@@ -13,14 +13,18 @@
 // (warp_strip.cuh); the lane keeps the integers of the last three rows'
 // windows in registers.  The warp checks each row against the current unit
 // with one vote and, when it does not fit, picks a unit for the last three
-// rows; output rows whose three rows share none (values near zero beside large ones,
-// infinities, NaN) take the per-pixel double-float form (terrain_px.cuh).
+// rows.  Output rows whose three rows share none (values through zero, several
+// binades of relief) are formed in 64-bit integers of up to 35 binades, TRI and
+// TPI rounded once, the curvature from its exact sums in FP64; rows with more
+// binades, infinities or NaN pixel by pixel (terrain_px.cuh).
 //
-// One conversion to float64 per TRI and TPI runs on the FP64 pipe (two
-// operations per clock and SM) beside the integer work; with the curvature's
-// conversions there too, that pipe would be the bound.  Bound by instruction
-// issue (about 100 per pixel), close to HBM (28 B/px with three float64
-// outputs).
+// One conversion to float64 per TRI and TPI runs on the narrow FP64 pipe beside
+// the integer work; with the curvature's conversions there too, that pipe would
+// be the bound.  Bound by instruction issue (about 100 per pixel), close to HBM
+// (28 B/px with three float64 outputs).  9001 x 7201 with three float64 outputs:
+// 0 .. 4500 m 442 us, -500 .. 500 m (a quarter of the pixels in 64-bit rows)
+// 647; 4096 x 4097 white noise (all of them) 300; one pixel per thread in
+// double-float 1052, 1078 and 320.
 #include "terrain_px.cuh"
 #include "warp_strip.cuh"
 
@@ -29,43 +33,67 @@ namespace {
 
 constexpr int kTsCols = 126;
 constexpr int kTsDepth = 6;  // rows in shared memory
-// Binades of a unit: |n| < 2^27, or 2^28 where no value is negative: either
-// way differences stay below 2^28 and the sums of eight below 2^31.
-constexpr uint32_t kTsSpan = 4, kTsSpanPos = 5;
+// Blocks per SM (strips of 8 rows) from which the strips are used; with fewer,
+// one pixel per thread (terrain.cu) is faster.  us, pixels | strips: float32 of
+// 1000 .. 1500 m 300^2 6.2 | 15, 1024^2 16.6 | 18.5, 1230^2 22.8 | 20.6; int16
+// 725^2 8.3 | 14.6, 1230^2 16.8 | 18.6, 1449^2 22.7 | 20.7; float32 through zero
+// 1024^2 21 | 31, 1449^2 35 | 43, 2048^2 68 | 65.
+constexpr int kTsFew = 10;
 
-// float64 bits of s 2^e, e20 = e 2^20: s + 2^31 as the low word of 2^52 + .,
-// one FP64 subtraction.
-__device__ __forceinline__ uint64_t scaled_bits(int32_t s, uint32_t e20) {
-  const double d = __hiloint2double(0x43300000, s ^ static_cast<int32_t>(0x80000000u)) -
-                   (4503599627370496.0 + 2147483648.0);
-  return static_cast<uint64_t>(__double_as_longlong(
-      __hiloint2double(__double2hiint(d) + static_cast<int32_t>(s ? e20 : 0u), __double2loint(d))));
-}
-
-template <typename B>
-__device__ __forceinline__ B out_bits(uint64_t b64) {
-  if constexpr (sizeof(B) == 8) return b64;
-  else return __float_as_uint(static_cast<float>(__longlong_as_double(static_cast<long long>(b64))));
-}
-
-// A pixel whose window does not fit one unit.
-template <typename T>
-__device__ __noinline__ void slow_pixel(const T* __restrict__ src, const DerivParams& P, int64_t x, int64_t y) {
+// A pixel whose row triple does not share a unit.
+__device__ __forceinline__ void lone_pixel(const float* __restrict__ src, const DerivParams& P, int64_t x, int64_t y) {
   float z[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const int64_t gy = min(max(y + k / 3 - 1, int64_t(0)), P.H - 1), gx = min(max(x + k % 3 - 1, int64_t(0)), P.W - 1);
-    z[k] = static_cast<float>(__ldg(src + gy * P.pitch + gx));
+    z[k] = __ldg(src + gy * P.pitch + gx);
   }
-  deriv_pixel(z, static_cast<int64_t>(blockIdx.z) * P.out_band_stride + y * P.out_pitch + x, P);
+  deriv_pixel(z, window_unit(z), static_cast<int64_t>(blockIdx.z) * P.out_band_stride + y * P.out_pitch + x, P);
 }
 
-template <typename T, typename B>
+// An output row whose three rows share no 32-bit unit.  Where they share a
+// 64-bit one, ``e`` is its lowest exponent (values through zero, several
+// binades of relief); otherwise every pixel looks for a unit of its own.  Out of
+// line, as the 32-bit rows' loop is near the instruction cache's size.
+struct Row3 {
+  float t[4], m[4], b[4];
+};
+constexpr int kTsWide = 128 + 8;  // a row's 64-bit integers, from element 4
+__device__ __noinline__ void odd_row(const Row3 r, uint32_t e, long long* __restrict__ buf, uint32_t writes,
+                                     const float* __restrict__ src, int64_t xw, int64_t y, const DerivParams& P) {
+  const int lane = threadIdx.x;
+  if (!e) {
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j)
+      if (writes >> j & 1u) lone_pixel(src, P, xw + 32 * j + lane, y);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    buf[4 + 32 * j + lane] = wide_int(r.t[j], e);
+    buf[kTsWide + 4 + 32 * j + lane] = wide_int(r.m[j], e);
+    buf[2 * kTsWide + 4 + 32 * j + lane] = wide_int(r.b[j], e);
+  }
+  __syncwarp();
+  const int64_t o = static_cast<int64_t>(blockIdx.z) * P.out_band_stride + y * P.out_pitch + xw + lane;
+#pragma unroll 2
+  for (int j = 0; j < 4; ++j) {
+    long long n[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) n[k] = buf[k / 3 * kTsWide + 3 + 32 * j + lane + k % 3];
+    if (writes >> j & 1u) deriv_ints(n, static_cast<int>(e) - 150, o + 32 * j, P);
+  }
+  __syncwarp();
+}
+
+// CK: the curvature factors have an integer form.
+template <typename T, typename B, bool CK>
 __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, const __grid_constant__ DerivParams P,
                                                     const int strip) {
   constexpr bool kFloat = std::is_same<T, float>::value;
   __shared__ __align__(16) unsigned char ring[16 + RowRing<T, kTsDepth>::kBytes + 16];
   __shared__ int32_t nrow[128 + 8];  // a float row's integers, from element 4
+  __shared__ long long wide[kFloat ? 3 * kTsWide : 1];  // three rows' in 64 bits, where 32 do not hold them
   const int lane = threadIdx.x;
   src += static_cast<int64_t>(blockIdx.z) * P.band_stride;
   const int64_t xw = static_cast<int64_t>(blockIdx.x) * kTsCols - 1, ys = static_cast<int64_t>(blockIdx.y) * strip;
@@ -101,7 +129,7 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
   uint32_t dt[4] = {0, 0, 0, 0}, dm[4] = {0, 0, 0, 0};  // nodata at or beside a column, a bit per lane
   uint32_t e0 = 127;       // the unit: exponent of the lowest binade, 2^(e0 - 150)
   float scale = 8388608.0f;  // 2^(150 - e0)
-  uint32_t signs = 0x7fffffffu, span = kTsSpan;  // all ones: negative values do not fit
+  uint32_t signs = 0x7fffffffu, span = kTdSpan;  // all ones: negative values do not fit
   bool shared = !kFloat;     // the last three rows are in this unit
   float vt[4] = {0.0f, 0.0f, 0.0f, 0.0f}, vm[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // their values
 #pragma unroll 1
@@ -120,6 +148,7 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
       }
     }
     int32_t bl[4], bc[4], br[4];
+    uint32_t ew = 0;  // the 64-bit unit's lowest exponent, or 0
     if constexpr (kFloat) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] = nd[j] ? 0.0f : v[j];
@@ -138,8 +167,7 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
         }
       };
       if (!__all_sync(0xffffffffu, fits) || !shared) {
-        // a unit for the last three rows: 64 <= exponents <= 190 (scaled
-        // results are normal, infinities and NaNs fail)
+        // a unit for the last three rows (infinities and NaNs fail)
         uint32_t lo = 0xffffffffu, hi = 0u;
         bool neg = false;
 #pragma unroll
@@ -154,12 +182,13 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
           }
         }
         signs = __any_sync(0xffffffffu, neg) ? 0x7fffffffu : 0xffffffffu;
-        span = signs == 0xffffffffu ? kTsSpanPos : kTsSpan;
+        span = signs == 0xffffffffu ? kTdSpanPos : kTdSpan;
         hi = __reduce_max_sync(0xffffffffu, hi);
-        lo = hi ? __reduce_min_sync(0xffffffffu, lo) : 0x3f800000u;  // zeros only: any unit
-        hi = hi ? hi : lo;
-        const uint32_t el = lo >> 23, eh = hi >> 23;
-        shared = el >= 64u && eh <= 190u && eh - el < span;
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        const uint32_t el = hi ? lo >> 23 : 127u, eh = hi ? hi >> 23 : 127u;  // zeros only: any unit
+        const bool normal = el >= kTdExpMin && eh <= kTdExpMax;
+        shared = normal && eh - el < span;
+        ew = normal && !shared && eh - el < kTdSpanWide ? el : 0u;
         if (shared) {
           e0 = el - (span - 1 - (eh - el)) / 2;
           scale = __uint_as_float((277u - e0) << 23);
@@ -194,7 +223,7 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
     }
     if (i >= 2) {
       const int64_t y = ys + i - 2;
-      if (shared && P.ck.ok) {
+      if (shared) {
         const int u = kFloat ? static_cast<int>(e0) - 150 : 0;
         const uint32_t e20 = static_cast<uint32_t>(u - 3) << 20;
 #pragma unroll
@@ -202,25 +231,22 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
           const int32_t c = mc[j];
           const bool w = writes >> j & 1u;
           if (tri) {
-            const int32_t s = (abs(tl[j] - c) + abs(tc[j] - c)) + (abs(tr[j] - c) + abs(ml[j] - c)) +
-                              (abs(mr[j] - c) + abs(bl[j] - c)) + (abs(bc[j] - c) + abs(br[j] - c));
-            const B b = out_bits<B>(scaled_bits(s, e20));
+            const B b = out_bits<B>(scaled_bits(tri8_of(tl[j], tc[j], tr[j], ml[j], c, mr[j], bl[j], bc[j], br[j]), e20));
             if (w) tri[32 * j] = b;
           }
           if (tpi) {
-            const int32_t s = 8 * c - ((tl[j] + tc[j] + tr[j]) + (ml[j] + mr[j]) + (bl[j] + bc[j] + br[j]));
-            const B b = out_bits<B>(scaled_bits(s, e20));
+            const B b = out_bits<B>(scaled_bits(tpi8_of(tl[j], tc[j], tr[j], ml[j], c, mr[j], bl[j], bc[j], br[j]), e20));
             if (w) tpi[32 * j] = b;
           }
           if (curv) {
-            const B b = out_bits<B>(vsr_curv_bits(ml[j] + mr[j] - 2 * c, tc[j] + bc[j] - 2 * c, &P.ck, u));
+            const int32_t ca = ml[j] + mr[j] - 2 * c, cb = tc[j] + bc[j] - 2 * c;
+            const B b = out_bits<B>(CK ? vsr_curv_bits(ca, cb, &P.ck, u) : curv_bits_f64(ca, cb, u, P));
             if (w) curv[32 * j] = b;
           }
         }
-      } else {
-#pragma unroll 1
-        for (int j = 0; j < 4; ++j)
-          if (writes >> j & 1u) slow_pixel<T>(src, P, xw + 32 * j + lane, y);
+      } else if constexpr (kFloat) {
+        odd_row(Row3{{vt[0], vt[1], vt[2], vt[3]}, {vm[0], vm[1], vm[2], vm[3]}, {v[0], v[1], v[2], v[3]}}, ew, wide,
+                writes, src, xw, y, P);
       }
       // borders and windows that touch nodata, over what was just written
       const bool border = y == 0 || y == P.H - 1;
@@ -263,15 +289,19 @@ __global__ void __launch_bounds__(32) terrain_strip(const T* __restrict__ src, c
 template <typename T>
 int launch_ts(const void* dem, const DerivParams& P, int bands, cudaStream_t st) {
   const int64_t gx = (P.W + kTsCols - 1) / kTsCols;
+  if (gx * ((P.H + 7) / 8) * bands < kTsFew * static_cast<int64_t>(sm_count())) return -1;
   int strip = 64;
   while (strip > 8 && gx * ((P.H + strip - 1) / strip) * bands < 32 * static_cast<int64_t>(sm_count())) strip /= 2;
   const int64_t gy = (P.H + strip - 1) / strip;
   if ((P.H + 7) / 8 > 65535 || gy > 65535)
     return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the terrain-derivative grid");
   const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(bands));
-  if (P.out_dtype == VSR_F64)
-    terrain_strip<T, unsigned long long><<<grid, 32, 0, st>>>(static_cast<const T*>(dem), P, strip);
-  else terrain_strip<T, unsigned int><<<grid, 32, 0, st>>>(static_cast<const T*>(dem), P, strip);
+  const T* src = static_cast<const T*>(dem);
+  const bool f64 = P.out_dtype == VSR_F64;
+  if (f64 && P.ck.ok) terrain_strip<T, unsigned long long, true><<<grid, 32, 0, st>>>(src, P, strip);
+  else if (f64) terrain_strip<T, unsigned long long, false><<<grid, 32, 0, st>>>(src, P, strip);
+  else if (P.ck.ok) terrain_strip<T, unsigned int, true><<<grid, 32, 0, st>>>(src, P, strip);
+  else terrain_strip<T, unsigned int, false><<<grid, 32, 0, st>>>(src, P, strip);
   VSR_CUDA_TRY(cudaGetLastError());
   return VSR_OK;
 }
@@ -283,7 +313,8 @@ int run_terrain_strip(const void* dem, int dtype, const DerivParams& P, int band
     case VSR_U8: return launch_ts<uint8_t>(dem, P, bands, st);
     case VSR_I16: return launch_ts<int16_t>(dem, P, bands, st);
     case VSR_U16: return launch_ts<uint16_t>(dem, P, bands, st);
-    default: return launch_ts<float>(dem, P, bands, st);
+    case VSR_F32: return launch_ts<float>(dem, P, bands, st);
+    default: return -1;
   }
 }
 
