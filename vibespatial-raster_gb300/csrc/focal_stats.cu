@@ -232,6 +232,9 @@ __global__ void __launch_bounds__(kFsThreads) focal_stat_kernel(const FsArgs a) 
           reinterpret_cast<float*>(obase)[y * a.out_pitch + x] =
               ndc[r * kFsTX + c] ? static_cast<float>(a.nd_out)
                                  : (n ? vsr_std_f32(static_cast<uint64_t>(num), static_cast<uint32_t>(n)) : 0.0f);
+        } else if (kh * kw <= kRecipTaps) {  // as the strips of focal_std.cu
+          out_at(r, c, num ? __longlong_as_double(static_cast<long long>(vsr_s64_std(
+                                 static_cast<uint64_t>(num), 0, fs_recip(n), 31 - __clz(n)))) : 0.0);
         } else {
           out_at(r, c, n ? sqrt(static_cast<double>(num)) / n : 0.0);
         }

@@ -2,8 +2,7 @@
 // rasters, square windows of radius 1..7.
 //
 // The reference takes two float64 passes over every window (algebra.py:
-// 3104-3122).  An SM of a GB300 starts only two FP64 operations per clock, so
-// that form is bound by 150 FP64 operations per pixel at 7 x 7.  Here the
+// 3104-3122).  The FP64 pipe of a GB300's SM is narrow, so that form is bound by 150 FP64 operations per pixel at 7 x 7.  Here the
 // values of a warp's strip are written as integers in one unit (the unit of
 // the strip's smallest non-zero magnitude), so that sum x and sum x^2 are
 // exact, slide down the rows without drift, and n^2 var = n sum x^2 -
@@ -15,8 +14,8 @@
 // 2^32 / n units (most DEM strips: n = 49 and values above 64 m allow 670 m
 // of relief), two limbs of 25 (R <= 3), 24 or 23 bits when its exponents span
 // at most 26, 24 or 22 binades (limb sums stay below 2^31, products' below
-// 2^60).  Other strips (wider spans, infinities,
-// values below 2^-103) keep the two float64 passes.
+// 2^60).  Other strips (wider spans, infinities, values below 2^-103) keep the
+// two float64 passes.
 //
 // Layout: warp strips (warp_strip.cuh).  Per input row a lane adds the
 // entering and subtracts the leaving row of its 4 columns (the last 2R+1 rows
@@ -39,6 +38,12 @@ namespace {
 constexpr int kSdThreads = 32;  // one warp per block: blocks of unequal strips (one word, two limbs) balance best
 constexpr int kSdMaxR = 7;  // windows of at most kRecipTaps: a count fits a byte
 static_assert((2 * kSdMaxR + 1) * (2 * kSdMaxR + 1) <= kRecipTaps, "reciprocal table");
+
+// Strips of 16 rows per SM below which a raster counts as small: 8/16-bit ones
+// take the shared-memory kernel (focal_stats.cu; uint16 3 x 3 at 300^2 12 us, 23
+// in strips, 7 x 7 at 512^2 18 | 25, 725^2 no difference), float32 ones strips of
+// 8 rows (7 x 7 at 512^2 27 us, 45 in strips of 16).
+constexpr int kSdFew = 2;
 
 template <int R>
 struct SdGeom {
@@ -283,41 +288,78 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
 }
 
 // Two float64 passes per window (strips whose values span too many binades
-// for the integers, or hold infinities).
+// for the integers, or hold infinities), two output rows at a time: the first
+// pass adds up columns once per row, then 2R+1 columns per window; the second
+// visits every tap.  Bound by the narrow FP64 pipe: 2 (2R+1)^2 + 2 (2R+1)
+// operations a pixel (3 (2R+1)^2 with both passes over the taps).
+// ``col``, ``cnt``: 256 each, of the warp.
 template <int R>
-__device__ __noinline__ void slow_strip(const FsArgs& a, const SdStrip& S) {
+__device__ __noinline__ void slow_strip(const FsArgs& a, const SdStrip& S, double* __restrict__ col,
+                                        int* __restrict__ cnt) {
+  constexpr int kCols = SdGeom<R>::kCols, kHalo = 4 * SdGeom<R>::HL;
   const int lane = threadIdx.x & 31;
   const float* src = static_cast<const float*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride;
-  const float ndv = static_cast<float>(a.ndv);
-  for (int p = lane; p < SdGeom<R>::kCols * S.nout; p += 32) {
-    const int64_t x = S.xw + 4 * SdGeom<R>::HL + p % SdGeom<R>::kCols, y = S.ys + p / SdGeom<R>::kCols;
-    if (x >= a.W) continue;
-    auto tap = [&](int dy, int dx, double& v) -> bool {
-      const int64_t yy = y + dy, xx = x + dx;
-      if (yy < 0 || yy >= a.H || xx < 0 || xx >= a.W) return false;
-      const float f = __ldg(src + yy * a.pitch + xx);
-      v = f;
-      return !fs_is_nd<float>(f, a.kind, ndv) && f == f;
-    };
-    double sm = 0.0, m2 = 0.0, v;
-    int n = 0;
-    for (int dy = -R; dy <= R; ++dy)
-      for (int dx = -R; dx <= R; ++dx)
-        if (tap(dy, dx, v)) {
-          sm += v;
-          ++n;
+  const float ndq = S.ndq, ndv = static_cast<float>(a.ndv);  // (NaN values are invalid whatever the nodata value)
+  for (int i = 0; i < S.nout; i += 2) {
+    for (int c = lane; c < 256; c += 32) {
+      const int64_t x = S.xw + (c & 127), y = S.ys + i + (c >> 7);
+      double s = 0.0;
+      int n = 0;
+      if (x >= 0 && x < a.W && y < a.H) {
+        const float* p = src + y * a.pitch + x;
+#pragma unroll
+        for (int dy = -R; dy <= R; ++dy) {
+          const bool in = y + dy >= 0 && y + dy < a.H;
+          const float f = in ? __ldg(p + dy * a.pitch) : __int_as_float(0x7fffffff);
+          if ((f == f) & (f != ndq)) {
+            s += static_cast<double>(f);
+            ++n;
+          }
         }
-    if (n) {
-      const double mean = sm / n;
-      for (int dy = -R; dy <= R; ++dy)
-        for (int dx = -R; dx <= R; ++dx)
-          if (tap(dy, dx, v)) m2 = fma(v - mean, v - mean, m2);
+      }
+      col[c] = s;
+      cnt[c] = n;
     }
-    double out = n ? sqrt(m2 / n) : 0.0;
-    if (fs_is_nd<float>(__ldg(src + y * a.pitch + x), a.kind, ndv)) out = a.nd_out;
-    const int64_t o = static_cast<int64_t>(blockIdx.z) * a.out_band_stride + y * a.out_pitch + x;
-    if (a.out_dtype == VSR_F64) static_cast<double*>(a.dst)[o] = out;
-    else static_cast<float*>(a.dst)[o] = static_cast<float>(out);
+    __syncwarp();
+    const int rows = S.nout - i < 2 ? 1 : 2;
+    for (int p = lane; p < rows * kCols; p += 32) {
+      const int r = p >= kCols, c = p - r * kCols + kHalo;
+      const int64_t x = S.xw + c, y = S.ys + i + r;
+      if (x >= a.W) continue;
+      double sm = 0.0, m2 = 0.0;
+      int n = 0;
+#pragma unroll
+      for (int d = -R; d <= R; ++d) {
+        sm += col[128 * r + c + d];
+        n += cnt[128 * r + c + d];
+      }
+      const float* const centre = src + y * a.pitch + x;
+      if (n) {
+        const double mean = sm / n;
+        auto add = [&](float f) {
+          if ((f == f) & (f != ndq)) {
+            const double d = static_cast<double>(f) - mean;
+            m2 = fma(d, d, m2);
+          }
+        };
+        if (y >= R && y + R < a.H && x >= R && x + R < a.W) {
+#pragma unroll
+          for (int dy = -R; dy <= R; ++dy)
+#pragma unroll
+            for (int dx = -R; dx <= R; ++dx) add(__ldg(centre + dy * a.pitch + dx));
+        } else {
+          for (int dy = -R; dy <= R; ++dy)
+            for (int dx = -R; dx <= R; ++dx)
+              if (y + dy >= 0 && y + dy < a.H && x + dx >= 0 && x + dx < a.W) add(__ldg(centre + dy * a.pitch + dx));
+        }
+      }
+      double out = n ? sqrt(m2 / n) : 0.0;
+      if (fs_is_nd<float>(__ldg(centre), a.kind, ndv)) out = a.nd_out;
+      const int64_t o = static_cast<int64_t>(blockIdx.z) * a.out_band_stride + y * a.out_pitch + x;
+      if (a.out_dtype == VSR_F64) static_cast<double*>(a.dst)[o] = out;
+      else static_cast<float*>(a.dst)[o] = static_cast<float>(out);
+    }
+    __syncwarp();
   }
 }
 
@@ -392,7 +434,7 @@ __global__ void __launch_bounds__(kSdThreads, 16) fs_strip_std(const FsArgs a, c
     const int span = static_cast<int>(__float_as_uint(vabs) >> 23) - E;
     // 24 <= E: the scales below are normal floats; infinities have exponent 255
     if (E < 24 || E > 250 || span > 2 * G::kLB - 24 || __float_as_uint(vabs) >= 0x7f800000u) {
-      slow_strip<R>(a, S);
+      slow_strip<R>(a, S, reinterpret_cast<double*>(sd_smem), reinterpret_cast<int*>(sd_smem + 256 * 8));
       return;
     }
     S.u = E - 150;
@@ -415,6 +457,7 @@ int launch_strip_std(const FsArgs& a, int bands, cudaStream_t st) {
   using G = SdGeom<R>;
   constexpr int kLimbs = std::is_same<T, float>::value ? 2 : 1;
   const size_t smem = 128 * 8 + static_cast<size_t>(G::P) * kSdThreads * (16 * kLimbs + 4);
+  static_assert(kLimbs == 1 || 128 * 8 + G::P * kSdThreads * (16 * kLimbs + 4) >= 256 * 12, "slow_strip's columns");
   auto kern = fs_strip_std<R, T>;
   static KernelResidency residency;
   int per_sm = 0;
@@ -425,6 +468,10 @@ int launch_strip_std(const FsArgs& a, int bands, cudaStream_t st) {
   // 11 x 11: 178 us with that, 191 us with 16 blocks per SM
   int strip = 128;
   while (strip > 16 && gx * ((a.H + strip - 1) / strip) * bands < 32 * static_cast<int64_t>(sm_count())) strip /= 2;
+  if (gx * ((a.H + 15) / 16) * bands < kSdFew * static_cast<int64_t>(sm_count())) {
+    if (!std::is_same<T, float>::value) return -1;
+    strip = 8;
+  }
   const int64_t gy = (a.H + strip - 1) / strip;
   if (gy > 65535) return -1;
   const bool vin = aligned(a.src, 4 * sizeof(T)) && a.pitch % 4 == 0 && (bands == 1 || a.band_stride % 4 == 0);
