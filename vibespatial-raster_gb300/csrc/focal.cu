@@ -9,8 +9,8 @@
 //   runtime width), one row partial sum per kernel row (for accuracy) and
 //   16-byte broadcast weight loads.  The weight-sum pass runs only on tiles
 //   that touch the border or hold nodata; other tiles use the full sum.
-// * sep_strip    -- the Gaussian as two 1-D passes inside one CTA: the row
-//   sums are held in shared memory and the column pass reads them.
+// * sep_tile, sep_strip -- the Gaussian as two 1-D passes inside one CTA: the
+//   row sums are held in shared memory and the column pass reads them.
 //   Numerator and weight sum are both separable, so this equals the
 //   reference's dense k x k normalised correlation with weights outer(g, g) /
 //   sum in real arithmetic, border and nodata handling included.  Kernels of
@@ -325,12 +325,136 @@ struct SepArgs {
   int out_dtype;
   int64_t out_pitch;
   int64_t band_stride, out_band_stride;
-  int seg;  // rows per CTA
 };
 
+// ------------------------------------------------------------- sep_tile --
+// Separable Gaussian of int32 and float64 rasters (k <= 33, where sep_tile_wins)
+// and of one tap, within a 128 x 32 output tile: the staged tile's row pass goes
+// to shared memory, the column pass reads it.  Bound by shared-memory reads and
+// its barriers, but with 32 + k - 1 rows per CTA where a strip's segment has 64
+// + k - 1 or more, one after the other.
+constexpr int kSTW = 128, kSTH = 32;
+
+inline size_t sep_smem_bytes(int k) {
+  const int SH = kSTH + k - 1, SW = kSTW + k - 1;
+  // staged v*valid and valid, row-pass numerator and denominator, weights
+  return static_cast<size_t>(((2 * SH * padded_width(SW) + 3) & ~3) + 2 * SH * kSTW + ((k + 3) & ~3)) * 4 + 16;
+}
+
+template <int MAXK>
+__global__ void __launch_bounds__(256) sep_tile(const SepArgs a) {
+  extern __shared__ __align__(16) float smem[];
+  const int k = a.k, r = k / 2;
+  const int SH = kSTH + k - 1, SW = kSTW + k - 1, PW = padded_width(SW);
+  float* vz = smem;
+  float* vd = vz + SH * PW;
+  float* rn = vz + ((2 * SH * PW + 3) & ~3);  // SH x kSTW row-pass numerator (16-byte aligned)
+  float* rd = rn + SH * kSTW;
+  float* g = rd + SH * kSTW;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t x0 = static_cast<int64_t>(blockIdx.x) * kSTW;
+  const int64_t y0 = static_cast<int64_t>(blockIdx.y) * kSTH;
+  const void* src = band_src(a.src, a.dtype, a.band_stride);
+  void* dst = band_dst(a.dst, a.out_dtype, a.out_band_stride);
+
+  for (int i = tid; i < k; i += 256) g[i] = a.g32[i];
+  for (int i = tid; i < SH * SW; i += 256) {
+    const int rr = i / SW, c = i - rr * SW;
+    const int64_t gy = y0 + rr - r, gx = x0 + c - r;
+    float v = 0.0f, d = 0.0f;
+    if (gy >= 0 && gy < a.H && gx >= 0 && gx < a.W) {
+      bool ok;
+      const float x = load_elem(src, a.dtype, gy * a.pitch + gx, a.nd, ok);
+      v = x * (ok ? 1.0f : 0.0f);
+      d = ok ? 1.0f : 0.0f;
+    }
+    vz[rr * PW + pos(c)] = v;
+    vd[rr * PW + pos(c)] = d;
+  }
+  __syncthreads();
+
+  // Row pass: each lane 4 adjacent columns of one staged row.
+  for (int rr = warp; rr < SH; rr += 8) {
+    const int c0 = 4 * lane;
+#pragma unroll
+    for (int plane = 0; plane < 2; ++plane) {
+      const float* row = (plane == 0 ? vz : vd) + rr * PW;
+      float V[4 + MAXK - 1];
+#pragma unroll
+      for (int j = 0; j < 4 + MAXK - 1; ++j) V[j] = (j < 4 + k - 1) ? row[pos(c0 + j)] : 0.0f;
+      float acc[4] = {};
+#pragma unroll
+      for (int t = 0; t < MAXK; ++t) {
+        if (t >= k) break;
+        const float w = g[t];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fmaf(w, V[u + t], acc[u]);
+      }
+      float* o = (plane == 0 ? rn : rd) + rr * kSTW + c0;
+      *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+  }
+  __syncthreads();
+
+  // Column pass: each thread one column, 16 consecutive output rows.
+  constexpr int RY = kSTH / 2;
+  const int c = tid & (kSTW - 1);
+  const int q0 = (tid >> 7) * RY;
+  float num[RY] = {}, den[RY] = {};
+#pragma unroll
+  for (int plane = 0; plane < 2; ++plane) {
+    const float* P = plane == 0 ? rn : rd;
+    float* acc = plane == 0 ? num : den;
+    for (int i = 0; i < RY + k - 1; ++i) {
+      const float v = P[(q0 + i) * kSTW + c];
+#pragma unroll
+      for (int ry = 0; ry < RY; ++ry) {
+        const int t = i - ry;
+        if (t >= 0 && t < k) acc[ry] = fmaf(g[t], v, acc[ry]);
+      }
+    }
+  }
+  const int64_t x = x0 + c;
+  if (x < a.W) {
+#pragma unroll
+    for (int ry = 0; ry < RY; ++ry) {
+      const int64_t y = y0 + q0 + ry;
+      if (y >= a.H) break;
+      const bool centre_ok = vd[(q0 + ry + r) * PW + pos(c + r)] != 0.0f;
+      const double out = (centre_ok && den[ry] > 0.0f) ? static_cast<double>(num[ry] / den[ry]) : a.nd_out;
+      store_out(dst, a.out_dtype, y * a.out_pitch + x, out);
+    }
+  }
+}
+
+template <int MAXK>
+int launch_sep(const SepArgs& a, cudaStream_t st, int bands = 1) {
+  const size_t smem = sep_smem_bytes(a.k);
+  auto kern = sep_tile<MAXK>;
+  VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  dim3 grid(static_cast<unsigned>((a.W + kSTW - 1) / kSTW), static_cast<unsigned>((a.H + kSTH - 1) / kSTH), bands);
+  if (grid.y > 65535u) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the separable Gaussian grid");
+  kern<<<grid, 256, smem, st>>>(a);
+  VSR_CUDA_TRY(cudaGetLastError());
+  return VSR_OK;
+}
+
+// Where sep_tile is faster than the strips.  us, tile | strips: one tap of
+// float32 400^2 19 | 24, 3000^2 103 | 84, of float64 3000^2 134 | 238; 5 taps of
+// int32 300^2 23 | 40, 8000^2 894 | 1544; 9 taps 850^2 31 | 42, 1230^2 48 | 46,
+// 2500^2 138 | 123, 5000^2 564 | 612; 17 taps 850^2 43 | 47, 1230^2 65 | 54; 33
+// taps 512^2 49 | 58, 850^2 89 | 58.
+bool sep_tile_wins(int dtype, int k, int64_t H, int64_t W, int bands) {
+  const int64_t tiles = ((W + kSTW - 1) / kSTW) * ((H + kSTH - 1) / kSTH) * bands, sms = sm_count();
+  if (dtype != VSR_I32 && dtype != VSR_F64) return k == 1 && tiles < 2 * sms;
+  if (k <= 5) return true;
+  if (k <= 17) return tiles < 2 * sms || (k <= 11 && tiles >= (dtype == VSR_F64 ? 12 : 16) * sms);
+  return k <= 33 && 2 * tiles < sms;
+}
+
 // ------------------------------------------------------------ sep_strip --
-// Separable Gaussian for what gauss_warp.cu does not take (k >= 19, int32 and
-// float64 rasters): a CTA walks a 128-column strip down a segment of rows.  Every input row is reduced
+// Separable Gaussian for what gauss_warp.cu and sep_tile do not take: a CTA
+// walks a 128-column strip down a segment of rows.  Every input row is reduced
 // along x once (row pass) into a ring of the last k + 15 row results; every
 // 16 new rows the column pass combines k ring rows into 16 output rows.
 // Numerator (v * valid) and weight sum (valid) travel together as float2
@@ -438,7 +562,7 @@ __device__ __forceinline__ float2 strip_tap(const void* src, int dtype, int64_t 
 }
 
 template <int DT, int KB>
-__global__ void __launch_bounds__(256, 2) sep_strip(const SepArgs a) {
+__global__ void __launch_bounds__(256, 2) sep_strip(const SepArgs a, const int seg) {  // seg: rows per CTA
   extern __shared__ __align__(16) float2 ssm2[];
   const int k = a.k, r = k / 2;
   const int NR = strip_nr(k);
@@ -450,8 +574,8 @@ __global__ void __launch_bounds__(256, 2) sep_strip(const SepArgs a) {
   uint32_t* vbits = reinterpret_cast<uint32_t*>(g2 + k8);  // NR x 8 words: staged-column validity bits
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t x0 = static_cast<int64_t>(blockIdx.x) * kSTW2;
-  const int64_t ys = static_cast<int64_t>(blockIdx.y) * a.seg;
-  const int64_t ye = min(ys + a.seg, a.H);
+  const int64_t ys = static_cast<int64_t>(blockIdx.y) * seg;
+  const int64_t ye = min(ys + seg, a.H);
   const void* src = band_src(a.src, a.dtype, a.band_stride);
   void* dst = band_dst(a.dst, a.out_dtype, a.out_band_stride);
   for (int i = tid; i < k8; i += 256) {
@@ -591,7 +715,7 @@ __global__ void __launch_bounds__(256, 2) sep_strip(const SepArgs a) {
   }
 }
 
-int launch_strip(SepArgs a, cudaStream_t st, int bands) {
+int launch_strip(const SepArgs& a, cudaStream_t st, int bands) {
   const size_t smem = strip_smem_bytes(a.k);
   if (smem > 227 * 1024) return fail(VSR_ERR_UNSUPPORTED, "Gaussian kernel %d too large for the strip kernel", a.k);
   // the taps of k in 65..72 (sigma 8 at 4 sigma) are unrolled; other k run-time
@@ -600,15 +724,26 @@ int launch_strip(SepArgs a, cudaStream_t st, int bands) {
               : a.dtype == VSR_F32 ? (k9 ? sep_strip<VSR_F32, 9> : sep_strip<VSR_F32, 0>)
                                    : (k9 ? sep_strip<0, 9> : sep_strip<0, 0>);
   VSR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  // two CTAs per SM: halve the segments until there are two rounds of them
-  // (a segment reads k - 1 rows more than it writes)
+  // Rows per segment: a CTA's time is about seg + k + 20 rows (k - 1 of them
+  // read again by the next segment), that of m CTAs on an SM, two at a time,
+  // 2 m + 1 (3.5 for one), fitted to 19 to 65 taps at 160^2 to 8000^2.  us at
+  // 64 | 128 | 256 | 512 rows: 49 taps of float32 850^2 47 | 72 | 121 | 216,
+  // 2500^2 172 | 155 | 182 | 219, 5000^2 569 | 504 | 459 | 505.
   const int64_t cols = (a.W + kSTW2 - 1) / kSTW2;
-  a.seg = kSSEG;
-  while (a.seg > 64 && a.seg > 2 * a.k && cols * ((a.H + a.seg - 1) / a.seg) * bands < 4 * static_cast<int64_t>(sm_count()))
-    a.seg /= 2;
-  dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>((a.H + a.seg - 1) / a.seg), bands);
+  double best = 0.0;
+  int seg = kSSEG;
+  for (int rows = kSSEG; rows >= 64; rows /= 2) {
+    const double per_sm = static_cast<double>(cols * ((a.H + rows - 1) / rows) * bands) / sm_count();
+    const double m = per_sm > 4.0 ? per_sm : std::ceil(per_sm);
+    const double t = (rows + a.k + 20) * (m > 1.0 ? 2.0 * m + 1.0 : 3.5);
+    if (rows == kSSEG || t < best) {  // 512 rows unless 7 % are to be had
+      best = rows == kSSEG ? 0.93 * t : t;
+      seg = rows;
+    }
+  }
+  dim3 grid(static_cast<unsigned>(cols), static_cast<unsigned>((a.H + seg - 1) / seg), bands);
   if (grid.y > 65535u) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the Gaussian grid");
-  kern<<<grid, 256, smem, st>>>(a);
+  kern<<<grid, 256, smem, st>>>(a, seg);
   VSR_CUDA_TRY(cudaGetLastError());
   return VSR_OK;
 }
@@ -1536,6 +1671,11 @@ static int gaussian_impl(const void* src, int dtype, int bands, int64_t band_str
   VSR_CUDA_TRY(cudaGetLastError());
   SepArgs a{src, dtype, height, width, pitch, nd, g32, k, nodata, dst, out_dtype, out_pitch, band_stride,
             out_band_stride};
+  if (sep_tile_wins(dtype, k, height, width, bands)) {
+    if (k <= 8) return launch_sep<8>(a, st, bands);
+    if (k <= 16) return launch_sep<16>(a, st, bands);
+    return launch_sep<33>(a, st, bands);
+  }
   return launch_strip(a, st, bands);
 }
 
