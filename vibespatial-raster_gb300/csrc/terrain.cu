@@ -95,31 +95,6 @@ int launch_deriv(const void* src, const DerivParams& P, int bands, cudaStream_t 
   return VSR_OK;
 }
 
-// 100 / cx^2 and 100 / cy^2 to 106 bits as integers in one unit of 2^-s, the
-// larger in [2^59, 2^60).
-vsr_curv_k curvature_factors(double cx2, double cy2) {
-  vsr_curv_k k{};
-  const double qx = 100.0 / cx2, qy = 100.0 / cy2;
-  const double rx = std::fma(-qx, cx2, 100.0) / cx2, ry = std::fma(-qy, cy2, 100.0) / cy2;
-  int e = 0;
-  std::frexp(std::max(qx, qy), &e);
-  k.s = 60 - e;
-  // cell sizes whose factors are far apart, or near the ends of the exponent
-  // range (the scaled results would not be normal): no integer form
-  k.ok = std::isfinite(qx) && std::isfinite(qy) && std::min(qx, qy) >= std::ldexp(std::max(qx, qy), -14) &&
-         e > -400 && e < 400;
-  if (!k.ok) return k;
-  auto fixed = [&](double q, double r) {
-    return static_cast<int64_t>(std::ldexp(q, k.s)) + static_cast<int64_t>(std::llrint(std::ldexp(r, k.s)));
-  };
-  const int64_t mx = fixed(qx, rx), my = fixed(qy, ry);
-  k.xh = static_cast<int32_t>(mx >> 31);
-  k.xl = static_cast<int32_t>(mx & 0x7fffffff);
-  k.yh = static_cast<int32_t>(my >> 31);
-  k.yl = static_cast<int32_t>(my & 0x7fffffff);
-  return k;
-}
-
 }  // namespace
 }  // namespace vsr
 
@@ -172,7 +147,7 @@ extern "C" int vsr_terrain_derivatives_bands(const void* dem, int dtype, int ban
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   P.kx = 100.0 / P.cx2;
   P.ky = 100.0 / P.cy2;
-  P.ck = curvature_factors(P.cx2, P.cy2);
+  P.ck = vsr_curv_factors(P.cx2, P.cy2);
   const int rc = run_terrain_strip(dem, dtype, P, bands, st);
   if (rc >= 0) return rc;
   switch (dtype) {

@@ -9,10 +9,12 @@
 // the result: the float64 formula rounds five times.  No FP64 operation: an
 // SM starts two per clock.
 //
-// Plain C so that a host program can check it; CUDA includes it as device code.
+// Plain C so that the host test compiles it with gcc; CUDA includes it as device
+// code (the factors as host code).
 #ifndef VSR_TERRAIN_FIXED_H
 #define VSR_TERRAIN_FIXED_H
 
+#include <math.h>
 #include <stdint.h>
 
 #if defined(__CUDACC__)
@@ -25,8 +27,33 @@
 typedef struct {
   int32_t xh, xl, yh, yl;
   int32_t s;
-  int32_t ok;  // 0: the factors are more than 2^14 apart (the smaller would lose bits)
+  int32_t ok;  // 0: no integer form
 } vsr_curv_k;
+
+// 100 / cx2 and 100 / cy2 to 106 bits as integers in one unit of 2^-s, the
+// larger in [2^59, 2^60].  No integer form where the factors are more than 2^14
+// apart (the smaller would lose bits) or near the ends of the exponent range
+// (the scaled results would not be normal).
+static inline vsr_curv_k vsr_curv_factors(double cx2, double cy2) {
+  vsr_curv_k k = {0, 0, 0, 0, 0, 0};
+  const double qx = 100.0 / cx2, qy = 100.0 / cy2;
+  const double rx = fma(-qx, cx2, 100.0) / cx2, ry = fma(-qy, cy2, 100.0) / cy2;
+  const double most = qx > qy ? qx : qy, least = qx > qy ? qy : qx;
+  if (!(least > 0.0) || !(most < 1.0e300)) return k;
+  int e = 0;
+  frexp(most, &e);
+  k.s = 60 - e;
+  k.ok = least >= ldexp(most, -14) && e > -400 && e < 400;
+  if (!k.ok) return k;
+  const double tx = ldexp(qx, k.s), ty = ldexp(qy, k.s);  // (the smaller may have a fraction)
+  const int64_t mx = (int64_t)tx + (int64_t)llrint(tx - floor(tx) + ldexp(rx, k.s));
+  const int64_t my = (int64_t)ty + (int64_t)llrint(ty - floor(ty) + ldexp(ry, k.s));
+  k.xh = (int32_t)(mx >> 31);
+  k.xl = (int32_t)(mx & 0x7fffffff);
+  k.yh = (int32_t)(my >> 31);
+  k.yl = (int32_t)(my & 0x7fffffff);
+  return k;
+}
 
 VSR_TF_FN int vsr_tf_clz32(uint32_t v) {  // v != 0
 #if defined(__CUDA_ARCH__)
