@@ -460,13 +460,29 @@ int launch_pairs(const FsArgs& a, int bands, cudaStream_t st) {
   return VSR_OK;
 }
 
+// A raster of few blocks in the bits form takes the pairs form (64 x 16 tiles): a
+// block numbers its values and makes its passes, or compares the pairs of eight
+// tiles, one after the other.  us, pairs | bits, of int32-held values as the
+// pairs form's: 3 x 3, 16-bit with 12 values 300^2 10 | 23, 1449^2 25 | 29,
+// 2048^2 43 | 39; with 300 values 512^2 10 | 47, 1449^2 23 | 58, 2048^2 37 | 74;
+// 8-bit with 12 values 725^2 12 | 15, 1024^2 15 | 19, 1449^2 25 | 17; 5 x 5,
+// 16-bit with 300 values 300^2 14 | 99, 1024^2 28 | 130, with 12 values 725^2 23
+// | 23, 1449^2 58 | 31.
+template <int R, typename T>
+bool few_blocks(const FsArgs& a, int bands) {
+  using G = VyGeom<R, T>;
+  constexpr int kPerSm = R == 1 ? (G::kByte ? 2 : 4) : (G::kByte ? 0 : 1);
+  const int64_t gx = (a.W + G::kWarps * G::kCols - 1) / (G::kWarps * G::kCols), gy = (a.H + kVyStrip - 1) / kVyStrip;
+  return gx * gy * bands < kPerSm * static_cast<int64_t>(sm_count());
+}
+
 template <typename T>
 int dispatch_t(const FsArgs& a, int bands, cudaStream_t st) {
   const bool square = a.ry == a.rx;
   if constexpr (std::is_integral<T>::value && sizeof(T) <= 2) {
     if (square) switch (a.ry) {
-        case 1: return launch_bits<1, T>(a, bands, st);
-        case 2: return launch_bits<2, T>(a, bands, st);
+        case 1: return few_blocks<1, T>(a, bands) ? launch_pairs<T, 1>(a, bands, st) : launch_bits<1, T>(a, bands, st);
+        case 2: return few_blocks<2, T>(a, bands) ? launch_pairs<T, 2>(a, bands, st) : launch_bits<2, T>(a, bands, st);
         case 3: return launch_bits<3, T>(a, bands, st);
         case 4: return launch_bits<4, T>(a, bands, st);
         case 5: return launch_bits<5, T>(a, bands, st);
