@@ -23,6 +23,7 @@
 #include <type_traits>
 #include <cmath>
 
+#include "mean_round.h"
 #include "vsr_internal.cuh"
 
 namespace vsr {
@@ -1234,7 +1235,7 @@ __global__ void __launch_bounds__(kSlTW) box_slide_int(const BoxArgs a) {
 constexpr int kBwLanes = 30;            // output lanes per warp
 constexpr int kBwCols = 4 * kBwLanes;   // output columns per warp
 constexpr int kBwWarps = 4;             // warps per block, side by side
-constexpr int kBwStrip = 256;           // output rows per warp
+constexpr int kBwStrip = 256;           // output rows per warp, fewer on small rasters
 
 template <typename T>
 struct Vec4Of {  // 4 elements in one load
@@ -1245,8 +1246,17 @@ struct Vec4Of<uint8_t> {
   using type = uint32_t;
 };
 
+template <bool F64>
+using CountPair = std::conditional_t<F64, double2, float2>;
+
+// An integer as a double: the low word of 2^52 + 2^31 + ., one FP64 subtraction.
+__device__ __forceinline__ double small_double(int v) {
+  return __hiloint2double(0x43300000, v ^ static_cast<int>(0x80000000u)) - (4503599627370496.0 + 2147483648.0);
+}
+
 template <int R, typename T, bool VOUT, bool F64, bool EDGE>
-__device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __restrict__ tab, int64_t xw) {
+__device__ __forceinline__ void box_strip(const BoxArgs& a, int strip, const CountPair<F64>* __restrict__ tab,
+                                          int64_t xw) {
   using Pk = SlidePack<R>;
   using V4 = typename Vec4Of<T>::type;
   constexpr int P = 2 * R + 1;
@@ -1257,21 +1267,30 @@ __device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __rest
   constexpr uint32_t kFlip = OFF ? 0x80008000u : 0u;
   const int lane = threadIdx.x & 31;
   const int64_t xs = xw - 4 + 4 * lane;  // this lane's first column (a multiple of 4)
-  const int64_t ys = static_cast<int64_t>(blockIdx.y) * kBwStrip;
+  const int64_t ys = static_cast<int64_t>(blockIdx.y) * strip;
   const T* src = static_cast<const T*>(band_src(a.src, a.dtype, a.band_stride));
   void* dst = band_dst(a.dst, a.out_dtype, a.out_band_stride);
-  const int nout = static_cast<int>(a.H - ys < kBwStrip ? a.H - ys : kBwStrip);
+  const int nout = static_cast<int>(a.H - ys < strip ? a.H - ys : static_cast<int64_t>(strip));
   const int nin = nout + 2 * R;  // input rows ys - R .. ys + nout + R - 1
   // input rows [r0, r1) lie in the raster
   const int r0 = ys < R ? static_cast<int>(R - ys) : 0;
   const int r1 = a.H - (ys - R) < nin ? static_cast<int>(a.H - (ys - R)) : nin;
-  // the nodata value as a packed word; no word equals 0xFFFFFFFF
+  // 8-bit: nodata in every byte; 16-bit: as a packed word (no word equals
+  // 0xFFFFFFFF).  One compare for 4 bytes, one compare and select per 16-bit
+  // element: uint8 7 x 7 at 7761 x 7264 123 us with the latter, 117 so; uint16
+  // the other way round (12 bands of 10980^2: 2192 | 1882)
+  const bool has_nd = a.nd.kind == VSR_NODATA_VALUE;
+  const uint32_t nd4 = (static_cast<uint32_t>(a.nd.iv) & 0xFFu) * 0x01010101u;
   const uint32_t ndw = a.nd.kind == VSR_NODATA_VALUE
                            ? kOne | ((static_cast<uint32_t>(a.nd.iv) ^ (kFlip & 0xFFFFu)) & (kByte ? 0xFFu : 0xFFFFu))
                            : 0xFFFFFFFFu;
   bool in[4];
+  uint32_t in4 = 0;  // the same, a byte each
 #pragma unroll
-  for (int e = 0; e < 4; ++e) in[e] = xs + e >= 0 && xs + e < a.W;
+  for (int e = 0; e < 4; ++e) {
+    in[e] = xs + e >= 0 && xs + e < a.W;
+    in4 |= in[e] ? 0xFFu << (8 * e) : 0u;
+  }
   const bool out_lane = lane >= 1 && lane <= kBwLanes && in[0];
   const bool vec = VOUT && in[3];
 
@@ -1298,7 +1317,7 @@ __device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __rest
   for (int u = 0; u < P; ++u) pre[u] = load(u, rp + u * a.pitch);
   const T* lp = rp + P * a.pitch;  // the row P ahead
   uint32_t hs[P][4];  // horizontal sums of the last P rows (ring slot = row % P)
-  uint32_t vm[P];     // their validity: byte e holds element e's count bit
+  uint32_t vm[P];     // their validity: byte e holds element e's count bit (16-bit) or is all ones (8-bit)
 #pragma unroll
   for (int u = 0; u < P; ++u) {
     vm[u] = 0u;
@@ -1312,10 +1331,11 @@ __device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __rest
   // correctly rounded sum / count for two columns: q0 = fs / n by the
   // reciprocal, one FMA residual correction (exact integers in float32)
   auto quot2 = [&](uint32_t va, uint32_t vb) -> float2 {
-    const float2 ta = tab[va >> Pk::kShift], tb = tab[vb >> Pk::kShift];
+    const CountPair<F64> ta = tab[va >> Pk::kShift], tb = tab[vb >> Pk::kShift];  // (called for float32 outputs)
     float2 fs = __fadd2_rn(make_float2(__uint_as_float(0x4B000000u | (va & kLow)), __uint_as_float(0x4B000000u | (vb & kLow))),
                            make_float2(-8388608.0f, -8388608.0f));
-    const float2 rn = make_float2(ta.x, tb.x), nn = make_float2(ta.y, tb.y);
+    const float2 rn = make_float2(static_cast<float>(ta.x), static_cast<float>(tb.x));
+    const float2 nn = make_float2(static_cast<float>(ta.y), static_cast<float>(tb.y));
     if (OFF) fs = __ffma2_rn(make_float2(static_cast<float>(OFF), static_cast<float>(OFF)), nn, fs);
     const float2 q0 = __fmul2_rn(fs, rn);
     return __ffma2_rn(__ffma2_rn(q0, nn, fs), rn, q0);
@@ -1333,28 +1353,33 @@ __device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __rest
       uint32_t w[12];  // left neighbour's 4 words, this lane's, the right neighbour's
       if (i >= r0 && i < r1) {
         if constexpr (kByte) {
-          w[4] = __byte_perm(raw, kOne, 0x7640);
-          w[5] = __byte_perm(raw, kOne, 0x7641);
-          w[6] = __byte_perm(raw, kOne, 0x7642);
-          w[7] = __byte_perm(raw, kOne, 0x7643);
+          uint32_t k = EDGE ? in4 : 0xFFFFFFFFu;
+          if (has_nd) k &= ~__vcmpeq4(raw, nd4);
+          vm[u] = k;
+          w[4] = __byte_perm(raw, kOne, 0x7640) & __byte_perm(k, 0u, 0x0000);
+          w[5] = __byte_perm(raw, kOne, 0x7641) & __byte_perm(k, 0u, 0x1111);
+          w[6] = __byte_perm(raw, kOne, 0x7642) & __byte_perm(k, 0u, 0x2222);
+          w[7] = __byte_perm(raw, kOne, 0x7643) & __byte_perm(k, 0u, 0x3333);
         } else {
           const uint32_t x = raw.x ^ kFlip, y = raw.y ^ kFlip;  // (v0 | v1 << 16), (v2 | v3 << 16)
           w[4] = __byte_perm(x, kOne, 0x7610);
           w[5] = __byte_perm(x, kOne, 0x7632);
           w[6] = __byte_perm(y, kOne, 0x7610);
           w[7] = __byte_perm(y, kOne, 0x7632);
-        }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          w[4 + e] = w[4 + e] == ndw ? 0u : w[4 + e];
-          if (EDGE) w[4 + e] = in[e] ? w[4 + e] : 0u;
+          for (int e = 0; e < 4; ++e) {
+            w[4 + e] = w[4 + e] == ndw ? 0u : w[4 + e];
+            if (EDGE) w[4 + e] = in[e] ? w[4 + e] : 0u;
+          }
         }
       } else {
+        vm[u] = 0u;
 #pragma unroll
         for (int e = 0; e < 4; ++e) w[4 + e] = 0u;
       }
       // the count bits (byte 2 of each word)
-      vm[u] = __byte_perm(__byte_perm(w[4], w[5], 0x0062), __byte_perm(w[6], w[7], 0x0062), 0x5410);
+      if constexpr (!kByte)
+        vm[u] = __byte_perm(__byte_perm(w[4], w[5], 0x0062), __byte_perm(w[6], w[7], 0x0062), 0x5410);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if (e >= 4 - R) w[e] = __shfl_up_sync(0xffffffffu, w[4 + e], 1);
@@ -1378,9 +1403,10 @@ __device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __rest
             for (int c = 0; c < 4; ++c) {
               const int cnt = static_cast<int>(V[c] >> Pk::kShift);
               const int sum = static_cast<int>(V[c] & kLow) - OFF * cnt;
+              const double2 t = tab[cnt];
               if (in[c])
                 reinterpret_cast<double*>(op)[c] =
-                    (cm & (kBit << (8 * c))) ? static_cast<double>(sum) / static_cast<double>(cnt) : a.nd_out;
+                    (cm & (kBit << (8 * c))) ? vsr_mean_quot(small_double(sum), t.y, t.x) : a.nd_out;
             }
           } else {
             const float2 q01 = quot2(V[0], V[1]), q23 = quot2(V[2], V[3]);
@@ -1401,31 +1427,42 @@ __device__ __forceinline__ void box_strip(const BoxArgs& a, const float2* __rest
   }
 }
 
-template <int R, typename T, bool VOUT, bool F64>
-__global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a) {
+// FULL: strips of kBwStrip rows, a constant (with ``rows``, 7 x 7 of 12 uint16
+// bands of 10980^2 takes 1934 us instead of 1873).
+template <int R, typename T, bool VOUT, bool F64, bool FULL>
+__global__ void __launch_bounds__(32 * kBwWarps) box_warp_int(const BoxArgs a, const int rows) {
   static_assert(R >= 1 && R <= 4, "the neighbour exchange covers radii up to 4");
   using Pk = SlidePack<R>;
   static_assert(Pk::kShift >= 16 && Pk::kShift <= 23, "the count bit sits in byte 2; value sums stay below 2^23");
-  __shared__ float2 tab[Pk::kTaps + 1];  // (RN(1/n), -n)
-  for (int i = threadIdx.x; i <= Pk::kTaps; i += blockDim.x)
-    tab[i] = make_float2(i ? __frcp_rn(static_cast<float>(i)) : 0.0f, -static_cast<float>(i));
+  __shared__ CountPair<F64> tab[Pk::kTaps + 1];  // (RN(1/n), -n)
+  for (int i = threadIdx.x; i <= Pk::kTaps; i += blockDim.x) {
+    if constexpr (F64) tab[i] = make_double2(i ? __drcp_rn(static_cast<double>(i)) : 0.0, -static_cast<double>(i));
+    else tab[i] = make_float2(i ? __frcp_rn(static_cast<float>(i)) : 0.0f, -static_cast<float>(i));
+  }
   __syncthreads();
   const int64_t xw = (static_cast<int64_t>(blockIdx.x) * kBwWarps + (threadIdx.x >> 5)) * kBwCols;
   if (xw >= a.W) return;  // the whole warp: no block-wide barrier follows
-  if (xw >= 4 && xw + 124 <= a.W) box_strip<R, T, VOUT, F64, false>(a, tab, xw);
-  else box_strip<R, T, VOUT, F64, true>(a, tab, xw);
+  const int strip = FULL ? kBwStrip : rows;
+  if (xw >= 4 && xw + 124 <= a.W) box_strip<R, T, VOUT, F64, false>(a, strip, tab, xw);
+  else box_strip<R, T, VOUT, F64, true>(a, strip, tab, xw);
 }
 
 template <int R, typename T>
 int launch_warp_t(const BoxArgs& a, cudaStream_t st, int bands) {
-  dim3 grid(static_cast<unsigned>((a.W + kBwWarps * kBwCols - 1) / (kBwWarps * kBwCols)),
-            static_cast<unsigned>((a.H + kBwStrip - 1) / kBwStrip), bands);
+  const int64_t gx = (a.W + kBwWarps * kBwCols - 1) / (kBwWarps * kBwCols);
+  // rows per warp: the most that gives every SM 16 blocks (2R rows of a strip are
+  // read again by the next one), from 256.  7 x 7 of uint16, us at 256 rows | at
+  // this rule: 1024^2 77 | 17, 4096^2 85 | 37, 10980^2 199 | 184
+  int strip = kBwStrip;
+  while (strip > 32 && gx * ((a.H + strip - 1) / strip) * bands < 16 * static_cast<int64_t>(sm_count())) strip /= 2;
+  dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>((a.H + strip - 1) / strip), bands);
   if (grid.y > 65535u) return fail(VSR_ERR_UNSUPPORTED, "raster too tall for the focal mean grid");
   const bool vout = a.out_dtype == VSR_F32 && aligned(a.dst, 16) && a.out_pitch % 4 == 0 &&
                     (bands == 1 || a.out_band_stride % 4 == 0);
-  if (a.out_dtype == VSR_F64) box_warp_int<R, T, false, true><<<grid, 32 * kBwWarps, 0, st>>>(a);
-  else if (vout) box_warp_int<R, T, true, false><<<grid, 32 * kBwWarps, 0, st>>>(a);
-  else box_warp_int<R, T, false, false><<<grid, 32 * kBwWarps, 0, st>>>(a);
+  if (a.out_dtype == VSR_F64) box_warp_int<R, T, false, true, false><<<grid, 32 * kBwWarps, 0, st>>>(a, strip);
+  else if (vout && strip == kBwStrip) box_warp_int<R, T, true, false, true><<<grid, 32 * kBwWarps, 0, st>>>(a, strip);
+  else if (vout) box_warp_int<R, T, true, false, false><<<grid, 32 * kBwWarps, 0, st>>>(a, strip);
+  else box_warp_int<R, T, false, false, false><<<grid, 32 * kBwWarps, 0, st>>>(a, strip);
   VSR_CUDA_TRY(cudaGetLastError());
   return VSR_OK;
 }

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kFsThreads) focal_stat_kernel(const FsArgs a) 
 constexpr int kFwLanes = 30;
 constexpr int kFwCols = 4 * kFwLanes;
 constexpr int kFwWarps = 4;
-constexpr int kFwStrip = 256;
+constexpr int kFwStrip = 256;  // output rows per warp, fewer on small rasters
 
 template <typename T>
 struct Fw4 {  // 4 elements in one load
@@ -297,7 +297,7 @@ struct Fw4<uint8_t> {
 };
 
 template <int R, typename T, int S, bool VOUT, bool F64>
-__global__ void __launch_bounds__(32 * kFwWarps) fs_warp_kernel(const FsArgs a) {
+__global__ void __launch_bounds__(32 * kFwWarps) fs_warp_kernel(const FsArgs a, const int strip) {
   static_assert(R >= 1 && R <= 4, "the neighbour exchange covers radii up to 4");
   static_assert(S == VSR_STAT_MIN || S == VSR_STAT_MAX || S == VSR_STAT_RANGE, "min, max or range");
   using V4 = typename Fw4<T>::type;
@@ -310,11 +310,11 @@ __global__ void __launch_bounds__(32 * kFwWarps) fs_warp_kernel(const FsArgs a) 
   const int64_t xw = (static_cast<int64_t>(blockIdx.x) * kFwWarps + (threadIdx.x >> 5)) * kFwCols;
   if (xw >= a.W) return;
   const int64_t xs = xw - 4 + 4 * lane;
-  const int64_t ys = static_cast<int64_t>(blockIdx.y) * kFwStrip;
+  const int64_t ys = static_cast<int64_t>(blockIdx.y) * strip;
   const T* src = static_cast<const T*>(a.src) + static_cast<int64_t>(blockIdx.z) * a.band_stride;
   char* obase = static_cast<char*>(a.dst) +
                 static_cast<int64_t>(blockIdx.z) * a.out_band_stride * (a.out_dtype == VSR_F64 ? 8 : 4);
-  const int nout = static_cast<int>(a.H - ys < kFwStrip ? a.H - ys : kFwStrip);
+  const int nout = static_cast<int>(a.H - ys < strip ? a.H - ys : static_cast<int64_t>(strip));
   const int nin = nout + 2 * R;
   const bool has_nd = a.kind == VSR_NODATA_VALUE;
   const uint32_t ndk = static_cast<uint32_t>(static_cast<int64_t>(a.ndv)) & kMask;  // nodata's bit pattern
@@ -457,15 +457,18 @@ __global__ void __launch_bounds__(32 * kFwWarps) fs_warp_kernel(const FsArgs a) 
 
 template <int R, typename T, int S>
 int fs_warp_launch(const FsArgs& a, int bands, cudaStream_t st) {
-  const dim3 grid(static_cast<unsigned>((a.W + kFwWarps * kFwCols - 1) / (kFwWarps * kFwCols)),
-                  static_cast<unsigned>((a.H + kFwStrip - 1) / kFwStrip), static_cast<unsigned>(bands));
+  const int64_t gx = (a.W + kFwWarps * kFwCols - 1) / (kFwWarps * kFwCols);
+  // rows per warp: the most that gives every SM 16 blocks, from 256 (as the mean)
+  int strip = kFwStrip;
+  while (strip > 32 && gx * ((a.H + strip - 1) / strip) * bands < 16 * static_cast<int64_t>(sm_count())) strip /= 2;
+  const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>((a.H + strip - 1) / strip), static_cast<unsigned>(bands));
   if (grid.y > 65535u) return -1;
   const bool vout = aligned(a.dst, a.out_dtype == VSR_F64 ? 32 : 16) && a.out_pitch % 4 == 0 &&
                     (bands == 1 || a.out_band_stride % 4 == 0);
-  if (a.out_dtype == VSR_F64 && vout) fs_warp_kernel<R, T, S, true, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
-  else if (a.out_dtype == VSR_F64) fs_warp_kernel<R, T, S, false, true><<<grid, 32 * kFwWarps, 0, st>>>(a);
-  else if (vout) fs_warp_kernel<R, T, S, true, false><<<grid, 32 * kFwWarps, 0, st>>>(a);
-  else fs_warp_kernel<R, T, S, false, false><<<grid, 32 * kFwWarps, 0, st>>>(a);
+  if (a.out_dtype == VSR_F64 && vout) fs_warp_kernel<R, T, S, true, true><<<grid, 32 * kFwWarps, 0, st>>>(a, strip);
+  else if (a.out_dtype == VSR_F64) fs_warp_kernel<R, T, S, false, true><<<grid, 32 * kFwWarps, 0, st>>>(a, strip);
+  else if (vout) fs_warp_kernel<R, T, S, true, false><<<grid, 32 * kFwWarps, 0, st>>>(a, strip);
+  else fs_warp_kernel<R, T, S, false, false><<<grid, 32 * kFwWarps, 0, st>>>(a, strip);
   VSR_CUDA_TRY(cudaGetLastError());
   return VSR_OK;
 }
