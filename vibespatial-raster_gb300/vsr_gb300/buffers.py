@@ -42,10 +42,13 @@ class RasterDiagnosticEvent:
 _EVENT_DEFAULTS = {f.name: f.default for f in fields(RasterDiagnosticEvent) if f.default is not MISSING}
 
 
-def diagnostic_event(kind, detail, residency, **given) -> RasterDiagnosticEvent:
+def diagnostic_event(kind, detail, residency, visible_to_user=False, elapsed_seconds=0.0) -> RasterDiagnosticEvent:
     """A RasterDiagnosticEvent without the per-field setattr of a frozen dataclass's __init__ (two per call)."""
     ev = object.__new__(RasterDiagnosticEvent)
-    ev.__dict__.update(_EVENT_DEFAULTS, kind=kind, detail=detail, residency=residency, **given)
+    d = ev.__dict__
+    d.update(_EVENT_DEFAULTS)
+    d["kind"], d["detail"], d["residency"] = kind, detail, residency
+    d["visible_to_user"], d["elapsed_seconds"] = visible_to_user, elapsed_seconds
     return ev
 
 
@@ -91,11 +94,11 @@ def _dtype_tables() -> _DtypeTables:
 
 
 def torch_dtype(np_dtype):
-    return _dtype_tables().torch_of[np.dtype(np_dtype)]
+    return (_TABLES or _dtype_tables()).torch_of[np.dtype(np_dtype)]
 
 
 def numpy_dtype(t_dtype) -> np.dtype:
-    return _dtype_tables().np_of[t_dtype]
+    return (_TABLES or _dtype_tables()).np_of[t_dtype]
 
 
 def _host_to_device(host: np.ndarray):
