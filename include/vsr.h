@@ -169,11 +169,13 @@ VSR_API int vsr_horn_fused_bands(const void* dem, int dtype, int bands, int64_t 
  * border pixels and pixels whose window touches nodata get ``nodata_out``
  * (the reference writes the raster's nodata, else -9999).  Outputs of
  * ``out_dtype`` (the reference returns float64), row pitch ``out_pitch``; any
- * of tri / tpi / curvature may be NULL.  8/16-bit DEMs, and float32 DEMs where
- * the values of three rows share a unit, are evaluated in integers (TRI and
- * TPI exact, the curvature a 96-bit product rounded once); other float32
- * windows in double-float FP32 (error-free differences, compensated sums: ~44
- * significant bits), int32 and float64 DEMs in FP64.
+ * of tri / tpi / curvature may be NULL.  8/16-bit and float32 DEMs are
+ * evaluated in integers where one unit holds the values (TRI and TPI exact,
+ * rounded once; the curvature a 96-bit product rounded once, or FP64 products
+ * of exact sums where the values span more than five binades or the cell sizes'
+ * squares are more than 2^14 apart), in double-float FP32 (~44 significant
+ * bits) where more than 35 binades, infinities or NaN come together; int32 and
+ * float64 DEMs in FP64.
  */
 VSR_API int vsr_terrain_derivatives(const void* dem, int dtype, int64_t height, int64_t width, int64_t pitch,
                                     double cell_x, double cell_y, double nodata, int nodata_kind,
@@ -316,9 +318,10 @@ VSR_API int vsr_focal_mean_bands(const void* src, int dtype, int bands, int64_t 
  *                        (non-nodata, non-NaN) taps, 0.0 for an empty window;
  *                        exact integer sums and sqrt(n^2 var)/n formed in
  *                        integers (within 0.52 ulp of float64) for 8/16-bit
- *                        rasters and for float32 ones where a strip's values
- *                        fit one unit, up to radius 7; two passes in float64
- *                        otherwise;
+ *                        rasters of windows up to 225 taps and for float32
+ *                        ones up to radius 7 where a strip's values fit one
+ *                        unit; wider 8/16-bit windows take the FP64 root of
+ *                        their exact sums, others two passes in float64;
  *   VSR_STAT_RANGE       max - min of the valid taps;
  *   VSR_STAT_VARIETY     number of distinct valid values, 0 for an empty
  *                        window (no cap; the reference GPU kernel stops at 49).

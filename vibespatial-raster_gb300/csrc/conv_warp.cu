@@ -14,7 +14,8 @@
 // all taps are valid; windows with a gap (nodata or the border) are summed
 // again over the validity bits of their rows.
 //
-// Bound by FMA issue from 7 x 7 on, by HBM and issue below.
+// Bound by instruction issue (5 x 5 at 4099 x 5003, 83 us: 77 % of the issue
+// slots, ALU pipe 55 %, FMA 32 %, DRAM 18 %).
 #include <cmath>
 
 #include "vsr_internal.cuh"

@@ -22,10 +22,12 @@
 // of integers wait in shared memory, each thread reading only its own), takes
 // the column sums of its neighbours by shuffles and adds up the window.
 //
-// Bound by instruction issue (about 150 per pixel, half of them the square
-// root and division).  7 x 7 on 4096^2: float32 151 us (8370 us with the two
-// float64 passes), uint16 128 us and 205 us with a float32 output (404 and
-// 586 us in 256-row strips of 128 threads with an FP64 root).
+// Bound by instruction issue and the latency of its chains (7 x 7 of float32
+// 4096^2: 61 % of the issue slots, ALU pipe 58 %, 14 warps per SM; about 200
+// instructions per pixel, half of them the square root and division).  7 x 7 on
+// 4096^2: float32 151 us (8370 us with the two float64 passes), uint16 128 us and
+// 205 us with a float32 output (404 and 586 us in 256-row strips of 128 threads
+// with an FP64 root).
 #include <cstring>
 
 #include "focal_stats.cuh"
@@ -40,9 +42,9 @@ constexpr int kSdMaxR = 7;  // windows of at most kRecipTaps: a count fits a byt
 static_assert((2 * kSdMaxR + 1) * (2 * kSdMaxR + 1) <= kRecipTaps, "reciprocal table");
 
 // Strips of 16 rows per SM below which a raster counts as small: 8/16-bit ones
-// take the shared-memory kernel (focal_stats.cu; uint16 3 x 3 at 300^2 12 us, 23
-// in strips, 7 x 7 at 512^2 18 | 25, 725^2 no difference), float32 ones strips of
-// 8 rows (7 x 7 at 512^2 27 us, 45 in strips of 16).
+// take the shared-memory kernel (focal_stats.cu; uint16 7 x 7 at 300 x 301 8 us,
+// 25 in strips), float32 ones strips of 8 rows (7 x 7 at 512^2 27 us, 45 in
+// strips of 16).
 constexpr int kSdFew = 2;
 
 template <int R>
@@ -291,7 +293,8 @@ __device__ __forceinline__ void run_strip(const FsArgs& a, const SdStrip& S, boo
 // for the integers, or hold infinities), two output rows at a time: the first
 // pass adds up columns once per row, then 2R+1 columns per window; the second
 // visits every tap.  Bound by the narrow FP64 pipe: 2 (2R+1)^2 + 2 (2R+1)
-// operations a pixel (3 (2R+1)^2 with both passes over the taps).
+// operations a pixel (3 (2R+1)^2 with both passes over the taps).  11 x 11 of
+// 3000 x 3001 values over 80 binades: 8.4 ms, 12.5 with both over the taps.
 // ``col``, ``cnt``: 256 each, of the warp.
 template <int R>
 __device__ __noinline__ void slow_strip(const FsArgs& a, const SdStrip& S, double* __restrict__ col,

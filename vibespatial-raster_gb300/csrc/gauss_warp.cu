@@ -19,7 +19,8 @@
 // arguments: FMAs read them from the constant bank, and the call is one
 // launch.
 //
-// Bound by instruction issue (FMA and shuffles), close to HBM.
+// Bound by instruction issue (13 taps at 6000^2, 162 us: 74 % of the issue slots,
+// ALU pipe 54 %, FMA 29 %, DRAM 21 %).
 #include <cmath>
 
 #include "vsr_internal.cuh"

@@ -8,10 +8,10 @@
 // arithmetic is horn_common.cuh's, two pixels per packed instruction: the
 // generic (scalar) kernel's results bit for bit, and the TMA kernel's.  float64
 // outputs are the float results widened by integer operations (a conversion
-// would occupy the FP64 pipe, two operations per clock and SM).
+// would occupy the narrow FP64 pipe).
 //
-// Bound by instruction issue and, with float64 outputs, HBM (19 B/px for
-// 16-bit DEMs).
+// Bound by instruction issue (int16 3601^2 with float64 outputs, 98 us: 68 % of
+// the issue slots, DRAM 24 %, 14 warps per SM).
 #include <type_traits>
 
 #include "horn_common.cuh"

@@ -1,8 +1,8 @@
 // sqrt(N) / n as a float64 with integer arithmetic, for the focal standard
 // deviation (N = n sum x^2 - (sum x)^2 formed exactly, std = sqrt(N) / n).
 //
-// An SM of a GB300 starts two FP64 operations per clock; a float64 square
-// root and a division take about 25 of them.  Here the root is a 64-bit
+// The FP64 pipe of a GB300's SM is narrow, and a float64 square root and a
+// division take about 25 operations on it.  Here the root is a 64-bit
 // fixed-point number: a float estimate, two Newton corrections whose
 // residuals are exact (mod 2^64) integer products, then one 64 x 64-bit
 // product with the reciprocal of n.  The error before the final rounding is
