@@ -462,18 +462,17 @@ int launch_pairs(const FsArgs& a, int bands, cudaStream_t st) {
 
 // A raster of few blocks in the bits form takes the pairs form (64 x 16 tiles): a
 // block numbers its values and makes its passes, or compares the pairs of eight
-// tiles, one after the other.  us, pairs | bits, of int32-held values as the
-// pairs form's: 3 x 3, 16-bit with 12 values 300^2 10 | 23, 1449^2 25 | 29,
-// 2048^2 43 | 39; with 300 values 512^2 10 | 47, 1449^2 23 | 58, 2048^2 37 | 74;
-// 8-bit with 12 values 725^2 12 | 15, 1024^2 15 | 19, 1449^2 25 | 17; 5 x 5,
-// 16-bit with 300 values 300^2 14 | 99, 1024^2 28 | 130, with 12 values 725^2 23
-// | 23, 1449^2 58 | 31.
+// tiles, one after the other.  us, pairs | bits: 3 x 3, 16-bit with 12 values
+// 300^2 10 | 21, 1449^2 25 | 29, 1740^2 33 | 29; with 250 values 512^2 9 | 47,
+// 1449^2 23 | 60; 8-bit with 12 values 725^2 10 | 15, 1024^2 17 | 17, 1230^2 21 |
+// 17, with 250 values 1024^2 14 | 47; 5 x 5, 16-bit with 250 values 300^2 13 | 73,
+// 725^2 19 | 74, with 12 values 725^2 23 | 23, 850^2 25 | 23.
 template <int R, typename T>
 bool few_blocks(const FsArgs& a, int bands) {
   using G = VyGeom<R, T>;
-  constexpr int kPerSm = R == 1 ? (G::kByte ? 2 : 4) : (G::kByte ? 0 : 1);
+  constexpr int kEighths = R == 1 ? (G::kByte ? 11 : 32) : (G::kByte ? 0 : 8);  // of a block per SM
   const int64_t gx = (a.W + G::kWarps * G::kCols - 1) / (G::kWarps * G::kCols), gy = (a.H + kVyStrip - 1) / kVyStrip;
-  return gx * gy * bands < kPerSm * static_cast<int64_t>(sm_count());
+  return 8 * gx * gy * bands < kEighths * static_cast<int64_t>(sm_count());
 }
 
 template <typename T>
